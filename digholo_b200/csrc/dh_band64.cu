@@ -225,8 +225,7 @@ __global__ void __launch_bounds__(NT, 1) k_band64(DhInvParams p, B64Args a) {
 
     const B64Smem L = band64Smem(PASS, w, G, GN);
     extern __shared__ float4 smf4[];
-    unsigned char* base = reinterpret_cast<unsigned char*>(
-        (reinterpret_cast<uintptr_t>(smf4) + 1023) & ~static_cast<uintptr_t>(1023));
+    unsigned char* base = tc::alignShared1024(reinterpret_cast<unsigned char*>(smf4));
     unsigned char* hiPlane = base + L.planes;                          // I8: [4][128][128 B]
     unsigned char* loPlane = hiPlane + (size_t)WF * 128;
     uint32_t* stage = reinterpret_cast<uint32_t*>(base + L.stage);    // [16][512] R | I << 16

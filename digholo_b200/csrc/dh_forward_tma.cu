@@ -32,6 +32,7 @@
 #include "dh_common.cuh"
 #include "dh_host.h"
 #include "dh_params.h"
+#include "dh_tc.cuh"
 #include "dh_twiddle128.h"
 
 using namespace dh;
@@ -218,8 +219,7 @@ __global__ void __launch_bounds__(256, 2) k_forward_tma(const __grid_constant__ 
 
     // shared layout: tiles (1024-aligned for the swizzle), column buffer
     // [H][w+1], exchange [HW][Q][w], tables, barriers
-    unsigned char* base = reinterpret_cast<unsigned char*>(
-        (reinterpret_cast<uintptr_t>(smRaw) + 1023) & ~static_cast<uintptr_t>(1023));
+    unsigned char* base = tc::alignShared1024(smRaw);
     unsigned char* tiles = base;
     float2* colbuf = reinterpret_cast<float2*>(tiles + (size_t)NBUF * tileBytes);
     constexpr int CLD = w + 1;

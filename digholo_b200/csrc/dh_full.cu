@@ -43,7 +43,7 @@ __global__ void __launch_bounds__(H * W / 32, 1) k_field_full(DhInvParams p) {
     unsigned char* sm = reinterpret_cast<unsigned char*>(smf4);
     // overlap operands first (1024-byte aligned for the 128-byte swizzle)
     unsigned char* base =
-        OVL ? reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(sm) + 1023) & ~static_cast<uintptr_t>(1023)) : sm;
+        OVL ? tc::alignShared1024(sm) : sm;
     constexpr uint32_t PB = OVL ? H * W * 2 : 0;    // one bf16 piece of one plane
     constexpr uint32_t BB = OVL ? GN * W * 2 : 0;   // one bf16 piece of Hx
     unsigned char* aHi = base;

@@ -12,6 +12,14 @@ namespace tc {
 
 __device__ __forceinline__ uint32_t sAddr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
+// Shared memory from its next 1024-byte boundary.  The offset is added to the
+// array itself: an address rounded as an integer and cast back is a generic
+// pointer, and every access through it a generic load or store (through the
+// global-memory queue) instead of a shared-memory one.
+__device__ __forceinline__ unsigned char* alignShared1024(unsigned char* sm) {
+    return sm + ((1024u - (sAddr(sm) & 1023u)) & 1023u);
+}
+
 __device__ __forceinline__ void mbarInitTc(uint64_t* bar) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sAddr(bar)) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
