@@ -180,18 +180,6 @@ struct B64Args {
     const unsigned char* hx;     // [pol][hi, lo][W / 128 atoms][GN][128 B] (swizzled bytes)
 };
 
-__device__ __forceinline__ uint32_t instrDescI8s(int M, int N, bool aSigned, bool bSigned) {
-    return (2u << 4) | ((aSigned ? 1u : 0u) << 7) | ((bSigned ? 1u : 0u) << 10) | ((uint32_t)(N >> 3) << 17) |
-           ((uint32_t)(M >> 4) << 24);
-}
-__device__ __forceinline__ void mmaI8(uint32_t dTmem, uint64_t aDesc, uint64_t bDesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(dTmem),
-        "l"(aDesc), "l"(bDesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
 __device__ __forceinline__ void tmemLoad16u(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
@@ -474,8 +462,8 @@ __global__ void __launch_bounds__(NT, 1) k_band64(DhInvParams p, B64Args a) {
         if (loaded) {
             const uint32_t aH = tc::sAddr(hiPlane), aL = tc::sAddr(loPlane);
             const uint32_t bH = tc::sAddr(hxHi), bL = tc::sAddr(hxLo);
-            const uint32_t dSS = instrDescI8s(128, GN, true, true), dSU = instrDescI8s(128, GN, true, false);
-            const uint32_t dUS = instrDescI8s(128, GN, false, true), dUU = instrDescI8s(128, GN, false, false);
+            const uint32_t dSS = tc::instrDescI8s(128, GN, true, true), dSU = tc::instrDescI8s(128, GN, true, false);
+            const uint32_t dUS = tc::instrDescI8s(128, GN, false, true), dUU = tc::instrDescI8s(128, GN, false, false);
             const uint32_t tHH = tmem, tMix = tmem + GN, tLL = tmem + 2 * GN;
 #pragma unroll
             for (int atom = 0; atom < WF / 128; atom++) {
@@ -484,10 +472,10 @@ __global__ void __launch_bounds__(NT, 1) k_band64(DhInvParams p, B64Args a) {
                     const uint32_t ao = (uint32_t)atom * 128 * 128 + (uint32_t)ks * 32;
                     const uint32_t bo = (uint32_t)atom * GN * 128 + (uint32_t)ks * 32;
                     const uint32_t acc = (atom > 0 || ks > 0) ? 1u : 0u;
-                    mmaI8(tHH, tc::smemDesc(aH + ao), tc::smemDesc(bH + bo), dSS, acc);
-                    mmaI8(tMix, tc::smemDesc(aH + ao), tc::smemDesc(bL + bo), dSU, acc);
-                    mmaI8(tMix, tc::smemDesc(aL + ao), tc::smemDesc(bH + bo), dUS, 1u);
-                    mmaI8(tLL, tc::smemDesc(aL + ao), tc::smemDesc(bL + bo), dUU, acc);
+                    tc::mmaI8(tHH, tc::smemDesc(aH + ao), tc::smemDesc(bH + bo), dSS, acc);
+                    tc::mmaI8(tMix, tc::smemDesc(aH + ao), tc::smemDesc(bL + bo), dSU, acc);
+                    tc::mmaI8(tMix, tc::smemDesc(aL + ao), tc::smemDesc(bH + bo), dUS, 1u);
+                    tc::mmaI8(tLL, tc::smemDesc(aL + ao), tc::smemDesc(bL + bo), dUU, acc);
                 }
             }
         } else if (p.status) {

@@ -1,11 +1,11 @@
-// Inverse stage for full-resolution fields (IFFTResolutionMode 0): the
-// Fourier window placed in the H x W plane -> IFFT -> field statistics ->
-// reference wave, -conj, int16 rounding (k_field_full), then the separable HG
-// overlap on the int16 field, either fused into k_field_full on the tensor
-// cores (split-BF16) or by k_overlap_f32 on the CUDA cores.  Same results as k_inverse in full-resolution mode and
-// as the reference's FFTW c2c backward digHolo.cpp:8734, digHoloFieldAnalysis
-// digHolo.cpp:2354, applyTilt16 digHolo.cpp:2701-2837 and
-// overlapFieldSeparable16 digHolo.cpp:2149-2341.
+// Inverse stage for full-resolution fields of 32 and 64 pixels
+// (IFFTResolutionMode 0; 128-pixel fields: dh_field128.cu): the Fourier
+// window placed in the H x W plane -> IFFT -> field statistics -> reference
+// wave, -conj, int16 rounding (k_field_full); and the separable HG overlap of
+// int16 fields on the CUDA cores (k_overlap_f32).  Same results as k_inverse
+// in full-resolution mode and as the reference's FFTW c2c backward
+// digHolo.cpp:8734, digHoloFieldAnalysis digHolo.cpp:2354, applyTilt16
+// digHolo.cpp:2701-2837 and overlapFieldSeparable16 digHolo.cpp:2149-2341.
 //
 // Pruned IFFT: only the h x w window is non-zero.  Along y, the window rows
 // sit at row_j = (r0 + j) mod H; with y = (H/h) t + u the column transform
@@ -22,15 +22,13 @@
 #include "dh_host.h"
 #include "dh_params.h"
 #include "dh_fft.cuh"
-#include "dh_tc.cuh"
 
 using namespace dh;
 
 
-// W, H: FFT window (= field) size; WW: IFFT window size (h = w = WW);
-// OVL: fuse the split-BF16 tensor-core overlap (H = 128, maxMG <= GN).
+// W, H: FFT window (= field) size; WW: IFFT window size (h = w = WW).
 // blockDim.x = H * W / 32; one block per (frame, polarisation).
-template <int W, int H, int WW, bool OVL, int GN>
+template <int W, int H, int WW>
 __global__ void __launch_bounds__(H * W / 32, 1) k_field_full(DhInvParams p) {
     constexpr int LOG = ilog2F(WW);
     constexpr int TX = W / WW, TY = H / WW;
@@ -38,19 +36,8 @@ __global__ void __launch_bounds__(H * W / 32, 1) k_field_full(DhInvParams p) {
     constexpr int NT = H * W / 32;
     constexpr int ALD = WW + 1;                     // stage-1 buffer row stride (complex)
     constexpr int SLD = W + 8;                      // int16 staging row stride (elements)
-    constexpr int TLD = H + 1;
     extern __shared__ float4 smf4[];
-    unsigned char* sm = reinterpret_cast<unsigned char*>(smf4);
-    // overlap operands first (1024-byte aligned for the 128-byte swizzle)
-    unsigned char* base =
-        OVL ? tc::alignShared1024(sm) : sm;
-    constexpr uint32_t PB = OVL ? H * W * 2 : 0;    // one bf16 piece of one plane
-    constexpr uint32_t BB = OVL ? GN * W * 2 : 0;   // one bf16 piece of Hx
-    unsigned char* aHi = base;
-    unsigned char* aLo = aHi + PB;
-    unsigned char* bHi = aLo + PB;
-    unsigned char* bLo = bHi + BB;
-    float2* A = reinterpret_cast<float2*>(bLo + BB);                  // [H][ALD]
+    float2* A = reinterpret_cast<float2*>(smf4);                      // [H][ALD]
     short* sR = reinterpret_cast<short*>(A + H * ALD);                // [H][SLD]
     short* sI = sR + H * SLD;
     constexpr int TWLD = WW + 1;                    // padded: lanes with different u hit different banks
@@ -59,17 +46,11 @@ __global__ void __launch_bounds__(H * W / 32, 1) k_field_full(DhInvParams p) {
     float* xax = reinterpret_cast<float*>(tw2 + TX * TWLD);          // [W]
     int* refX = reinterpret_cast<int*>(xax + W);                      // [W] packed (xr, xi)
     StatF* red = reinterpret_cast<StatF*>(refX + W);                  // [NT / 32]
-    float* T = reinterpret_cast<float*>(red + NT / 32);               // OVL: [2][GN][TLD]
-    float* hy = T + (OVL ? 2 * GN * TLD : 0);                         // OVL: [G][TLD]
-    int* modeMN = reinterpret_cast<int*>(hy + (OVL ? p.maxMG * TLD : 0));
-    uint64_t* bar = reinterpret_cast<uint64_t*>(
-        (reinterpret_cast<uintptr_t>(modeMN + (OVL ? p.modeCount : 0)) + 7) & ~static_cast<uintptr_t>(7));
-    uint32_t* tmemSlot = reinterpret_cast<uint32_t*>(bar + 1);
 
     const int unit = blockIdx.x;
     const int P = p.polCount;
     const int pol = unit % P, frame = unit / P;
-    const int tid = threadIdx.x, warp = tid >> 5;
+    const int tid = threadIdx.x;
     const short* ref = p.refWave + (size_t)pol * 2 * (W + H);
     const int r0 = ((p.sy[pol] + H / 2) % H + H) % H;
     const int sx0 = p.sx0[pol];
@@ -87,35 +68,6 @@ __global__ void __launch_bounds__(H * W / 32, 1) k_field_full(DhInvParams p) {
         const int u = e / WW, k = e % WW;
         const int col = (sx0 + ((k - sx0) & (WW - 1))) & (W - 1);
         tw2[u * TWLD + k] = expPos(p.twiddle, col * u, W);
-    }
-    const int G = p.maxMG, M = p.modeCount;
-    if (OVL) {
-        // Hx of this polarisation as the B operand (rows m >= G zero), Hy, modes
-        for (int e = tid; e < GN * (W / 8); e += NT) {
-            const int m = e / (W / 8), q = e % (W / 8);
-            uint4 raw = make_uint4(0, 0, 0, 0);
-            if (m < G) raw = __ldg(reinterpret_cast<const uint4*>(p.hgX + ((size_t)pol * G + m) * W) + q);
-            uint4 hi, lo;
-            tc::split8(raw, hi, lo);
-            const uint32_t off = tc::swzOffset(GN, m, q);
-            *reinterpret_cast<uint4*>(bHi + off) = hi;
-            *reinterpret_cast<uint4*>(bLo + off) = lo;
-        }
-        for (int e = tid; e < G * H; e += NT) hy[(e / H) * TLD + (e % H)] = (float)p.hgY[(size_t)pol * G * H + e];
-        for (int mode = tid; mode < M; mode += NT) {
-            int g = (int)((sqrtf(8.0f * mode + 1.0f) - 1.0f) * 0.5f);
-            while ((g + 1) * (g + 2) / 2 <= mode) g++;
-            while (g * (g + 1) / 2 > mode) g--;
-            const int n = mode - g * (g + 1) / 2;
-            modeMN[mode] = ((g - n) << 16) | n;
-        }
-        if (tid == 0) tc::mbarInitTc(bar);
-        if (warp == 0) {
-            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 64;" ::"r"(tc::sAddr(tmemSlot)) : "memory");
-            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-        }
-        tc::fenceProxyAsync();
-        tc::fenceBeforeSync();
     }
     __syncthreads();
 
@@ -238,7 +190,7 @@ __global__ void __launch_bounds__(H * W / 32, 1) k_field_full(DhInvParams p) {
             sI[y * SLD + x] = roundSat16(scale * vi);
         }
     }
-    if (!OVL && p.fieldsOnly) return;   // block-uniform
+    if (p.fieldsOnly) return;   // block-uniform
     __syncthreads();
     // coalesced copy of the int16 planes
     constexpr int CH = W / 8;   // 16-byte chunks per row
@@ -248,88 +200,6 @@ __global__ void __launch_bounds__(H * W / 32, 1) k_field_full(DhInvParams p) {
         const int y = e / CH, q = e % CH;
         gR[e] = *reinterpret_cast<const uint4*>(sR + y * SLD + 8 * q);
         gI[e] = *reinterpret_cast<const uint4*>(sI + y * SLD + 8 * q);
-    }
-    if (!OVL) return;
-
-    // Fused overlap (digHolo.cpp:2149-2341) on the tensor cores, split-BF16:
-    // T[y][m] = sum_x V[y][x] Hx[m][x] per plane (hi.hi + hi.lo + lo.hi, FP32
-    // accumulation in tensor memory), then c_mn = sum_y Hy[n][y] T[y][m].
-    const uint32_t tmem = *tmemSlot;
-    constexpr uint32_t IDESC = tc::instrDesc(128, GN);
-    bool ok = true;
-    for (int plane = 0; plane < 2 && ok; plane++) {
-        const short* sp = plane ? sI : sR;
-        for (int e = tid; e < H * CH; e += NT) {
-            const int y = e / CH, q = e % CH;
-            uint4 hi, lo;
-            tc::split8(*reinterpret_cast<const uint4*>(sp + y * SLD + 8 * q), hi, lo);
-            const uint32_t off = tc::swzOffset(H, y, q);
-            *reinterpret_cast<uint4*>(aHi + off) = hi;
-            *reinterpret_cast<uint4*>(aLo + off) = lo;
-        }
-        tc::fenceProxyAsync();
-        __syncthreads();
-        if (tid == 0) {
-            tc::fenceAfterSync();
-            const uint32_t d = tmem + (uint32_t)(plane * GN);
-            const uint32_t aH = tc::sAddr(aHi), aL = tc::sAddr(aLo), bH = tc::sAddr(bHi), bL = tc::sAddr(bLo);
-#pragma unroll
-            for (int k = 0; k < W / 16; k++) {
-                const uint32_t ka = (uint32_t)(k >> 2) * H * 128 + (uint32_t)(k & 3) * 32;
-                const uint32_t kb = (uint32_t)(k >> 2) * GN * 128 + (uint32_t)(k & 3) * 32;
-                tc::mmaBf16(d, tc::smemDesc(aH + ka), tc::smemDesc(bH + kb), IDESC, k > 0 ? 1u : 0u);
-                tc::mmaBf16(d, tc::smemDesc(aH + ka), tc::smemDesc(bL + kb), IDESC, 1u);
-                tc::mmaBf16(d, tc::smemDesc(aL + ka), tc::smemDesc(bH + kb), IDESC, 1u);
-            }
-            tc::mmaCommit(bar);
-        }
-        // the operand buffer is rewritten for the next plane only after the MMAs finish
-        ok = !__syncthreads_or(!tc::mbarWaitTc(bar, (unsigned)plane));
-        tc::fenceAfterSync();
-    }
-    if (ok) {
-        if (warp < 4) {
-            const uint32_t rowAddr = tmem + ((uint32_t)(warp * 32) << 16);
-#pragma unroll
-            for (int pl = 0; pl < 2; pl++) {
-#pragma unroll
-                for (int c0 = 0; c0 < GN; c0 += 16) {
-                    float v[16];
-                    tc::tmemLoad16(rowAddr + (uint32_t)(pl * GN + c0), v);
-#pragma unroll
-                    for (int i = 0; i < 16; i++) T[(pl * GN + c0 + i) * TLD + tid] = v[i];
-                }
-            }
-        }
-        tc::fenceBeforeSync();
-        __syncthreads();
-        const float fieldScale = 1.0f / scale;
-        const float* sxp = p.hgScaleX + pol * G;
-        const float* syp = p.hgScaleY + pol * G;
-        for (int mode = tid; mode < M; mode += NT) {
-            const int mn = modeMN[mode];
-            const int m = mn >> 16, n = mn & 0xFFFF;
-            const float* hn = hy + n * TLD;
-            const float* tr = T + m * TLD;
-            const float* ti = T + (GN + m) * TLD;
-            float cr = 0.f, ci = 0.f;
-#pragma unroll 8
-            for (int yy = 0; yy < H; yy++) {
-                cr = fmaf(hn[yy], tr[yy], cr);
-                ci = fmaf(hn[yy], ti[yy], ci);
-            }
-            const float ms = (float)((double)sxp[m] * (double)syp[n] * (double)fieldScale);
-            p.coefs[(size_t)frame * P * M + (size_t)pol * M + mode] = make_float2(cr * ms, ci * ms);
-        }
-    } else if (tid == 0 && p.status) {
-        *(volatile int*)p.status = 2;
-        __threadfence_system();
-    }
-    tc::fenceBeforeSync();
-    __syncthreads();
-    if (warp == 0) {
-        tc::fenceAfterSync();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 64;" ::"r"(tmem) : "memory");
     }
 }
 
@@ -490,20 +360,17 @@ __global__ void __launch_bounds__(256) k_overlap_f32_chunked(DhInvParams p, int 
     }
 }
 
+cudaError_t dh_launch_field128(const DhInvParams& p, int withOverlap, cudaStream_t s);
+
 namespace {
 
-template <int W, int H, int WW, bool OVL, int GN>
+template <int W, int H, int WW>
 cudaError_t launchField(const DhInvParams& p, cudaStream_t s) {
     constexpr int NT = H * W / 32;
-    const size_t ovl = OVL ? 1024 + 2 * (size_t)H * W * 2 + 2 * (size_t)GN * W * 2 : 0;
-    const size_t tail = OVL ? sizeof(float) * (2 * (size_t)GN * (H + 1) + (size_t)p.maxMG * (H + 1)) +
-                                  sizeof(int) * (size_t)p.modeCount + 32
-                            : 0;
-    const size_t smem = ovl + sizeof(float2) * (size_t)H * (WW + 1) + sizeof(short) * 2 * (size_t)H * (W + 8) +
+    const size_t smem = sizeof(float2) * (size_t)H * (WW + 1) + sizeof(short) * 2 * (size_t)H * (W + 8) +
                         sizeof(float2) * (size_t)(H / WW + W / WW) * (WW + 1) + sizeof(float) * W + sizeof(int) * W +
-                        sizeof(StatF) * (NT / 32) + tail;
-    if (smem > 227 * 1024) return cudaErrorNotSupported;
-    auto kern = k_field_full<W, H, WW, OVL, GN>;
+                        sizeof(StatF) * (NT / 32);
+    auto kern = k_field_full<W, H, WW>;
     cudaError_t e = setSmemOnce(reinterpret_cast<const void*>(kern), (int)smem);
     if (e != cudaSuccess) return e;
     kern<<<(unsigned)(p.frameCount * p.polCount), NT, smem, s>>>(p);
@@ -522,31 +389,28 @@ cudaError_t launchOverlapF32(const DhInvParams& p, int nx, int ny, cudaStream_t 
 
 }  // namespace
 
-// Full-resolution field kernel; cudaErrorNotSupported outside its shapes.
-// withOverlap: fuse the split-BF16 tensor-core overlap (128-row fields,
-// maxMG <= 32); *fused reports whether it did.
+// Full-resolution field kernels up to 128 x 128; cudaErrorNotSupported
+// outside their shapes.  withOverlap: fuse the tensor-core overlap (128 x 128
+// fields, maxMG <= 32); *fused reports whether it did, or, beside
+// cudaErrorNotSupported, that the fields alone are supported.
 cudaError_t dh_launch_field_full(const DhInvParams& p, int withOverlap, int* fused, cudaStream_t s) {
     *fused = 0;
-    if (p.lowres || p.logw != p.logh || p.logW != p.logH) return cudaErrorNotSupported;
-    if (p.w != (1 << p.logw) || p.h != (1 << p.logh)) return cudaErrorNotSupported;   // power-of-two windows only
+    if (p.lowres || p.logW != p.logH) return cudaErrorNotSupported;
+    const bool pow2 = p.logw == p.logh && p.w == (1 << p.logw) && p.h == (1 << p.logh);
+    if (p.logW == 7) {
+        const int ovl = withOverlap && p.maxMG > 0 && p.coefs && p.maxMG <= 32;
+        const cudaError_t e = dh_launch_field128(p, ovl, s);
+        *fused = ovl && (e != cudaErrorNotSupported || pow2);
+        return e;
+    }
+    if (!pow2) return cudaErrorNotSupported;
     if (p.frameCount * p.polCount <= 0) return cudaSuccess;
     const int W = 1 << p.logW, w = 1 << p.logw;
-    const bool ovl = withOverlap && p.maxMG > 0 && p.coefs && p.maxMG <= 32 && W == 128;
-    if (ovl) {
-        *fused = 1;
-        const bool small = p.maxMG <= 16;
-        if (w == 16) return small ? launchField<128, 128, 16, true, 16>(p, s) : launchField<128, 128, 16, true, 32>(p, s);
-        if (w == 32) return small ? launchField<128, 128, 32, true, 16>(p, s) : launchField<128, 128, 32, true, 32>(p, s);
-        *fused = 0;
-        return cudaErrorNotSupported;
-    }
     if (w == 16) {
-        if (W == 128) return launchField<128, 128, 16, false, 16>(p, s);
-        if (W == 64) return launchField<64, 64, 16, false, 16>(p, s);
-        if (W == 32) return launchField<32, 32, 16, false, 16>(p, s);
+        if (W == 64) return launchField<64, 64, 16>(p, s);
+        if (W == 32) return launchField<32, 32, 16>(p, s);
     } else if (w == 32) {
-        if (W == 128) return launchField<128, 128, 32, false, 16>(p, s);
-        if (W == 64) return launchField<64, 64, 32, false, 16>(p, s);
+        if (W == 64) return launchField<64, 64, 32>(p, s);
     }
     return cudaErrorNotSupported;
 }

@@ -929,10 +929,13 @@ static cudaError_t launchInverse(Object& o, const DhInvParams& ip, bool mayAlloc
         if (e == cudaSuccess) { o.lastInverseKernel = 2; o.lastOverlapKernel = 1; return e; }
         if (e != cudaErrorNotSupported) return e;
         cudaGetLastError();
-        // full resolution: field kernel, then the overlap kernel
+        // full resolution: field kernel, then the overlap kernel (128 x 128
+        // fields with 48-pixel windows report the number of the band kernels,
+        // whose folded transforms they run)
+        const int fieldKernel = isPow2(ip.w) && isPow2(ip.h) ? 3 : 4;
         int fused = 0;
         e = dh_launch_field_full(ip, o.overlapKernel == 0, &fused, o.stream);
-        if (e == cudaSuccess && fused) { o.lastInverseKernel = 3; o.lastOverlapKernel = 2; return e; }
+        if (e == cudaSuccess && fused) { o.lastInverseKernel = fieldKernel; o.lastOverlapKernel = 2; return e; }
         if (e == cudaErrorNotSupported && fused) {
             cudaGetLastError();
             e = dh_launch_field_full(ip, 0, &fused, o.stream);
@@ -944,7 +947,7 @@ static cudaError_t launchInverse(Object& o, const DhInvParams& ip, bool mayAlloc
                 cudaGetLastError();
                 e = dh_launch_overlap_f32_chunked(ip, nx, ny, o.stream);
             }
-            if (e == cudaSuccess) { o.lastInverseKernel = 3; o.lastOverlapKernel = 1; return e; }
+            if (e == cudaSuccess) { o.lastInverseKernel = fieldKernel; o.lastOverlapKernel = 1; return e; }
             if (e != cudaErrorNotSupported) return e;
             cudaGetLastError();
             // overlap shape not covered: rerun the whole stage with another kernel

@@ -65,6 +65,19 @@ __device__ __forceinline__ void mmaBf16(uint32_t dTmem, uint64_t aDesc, uint64_t
         "l"(aDesc), "l"(bDesc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
+// kind::i8: 8-bit A and B (each signed or unsigned), int32 accumulator, K = 32.
+__host__ __device__ constexpr uint32_t instrDescI8s(int M, int N, bool aSigned, bool bSigned) {
+    return (2u << 4) | ((aSigned ? 1u : 0u) << 7) | ((bSigned ? 1u : 0u) << 10) | ((uint32_t)(N >> 3) << 17) |
+           ((uint32_t)(M >> 4) << 24);
+}
+__device__ __forceinline__ void mmaI8(uint32_t dTmem, uint64_t aDesc, uint64_t bDesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(dTmem),
+        "l"(aDesc), "l"(bDesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
 __device__ __forceinline__ void mmaCommit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(sAddr(bar))
                  : "memory");
@@ -95,6 +108,18 @@ __device__ __forceinline__ void tmemLoad16(uint32_t taddr, float (&v)[16]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
     for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
+}
+
+// 8 consecutive accumulator columns of this warp's 32 lanes; the values are
+// there after tmemWaitLoad8() on them.
+__device__ __forceinline__ void tmemLoad8(uint32_t taddr, uint32_t (&r)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr));
+}
+__device__ __forceinline__ void tmemWaitLoad8(uint32_t (&r)[8]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])::"memory");
 }
 
 // Exact split of 8 int16 values into bf16 hi and lo (element order kept).
