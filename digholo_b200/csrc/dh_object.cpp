@@ -33,6 +33,7 @@ cudaError_t dh_launch_field_band64(const DhInvParams& p, int overlapKind, void* 
                                    int* overlapUsed, cudaStream_t s);
 int dh_forward_i8_npad(int w);
 cudaError_t dh_launch_inverse_lo(const DhInvParams& p, cudaStream_t s);
+cudaError_t dh_launch_forward_win(const DhFwdParams& f, cudaStream_t s);
 cudaError_t dh_launch_field_full(const DhInvParams& p, int withOverlap, int* fused, cudaStream_t s);
 cudaError_t dh_launch_overlap_f32(const DhInvParams& p, int nx, int ny, cudaStream_t s);
 cudaError_t dh_launch_overlap_f32_chunked(const DhInvParams& p, int nx, int ny, cudaStream_t s);
@@ -814,9 +815,13 @@ static cudaError_t launchForward(Object& o, const DhFwdParams& fp, bool mayAlloc
         cudaGetLastError();
     }
     // windows of 256 pixels and more, and IFFT windows whose sides are not
-    // powers of two: through the full planes (the plane buffer of the
-    // Fourier-plane requests, batch-sized)
+    // powers of two: up to 256 x 256 in one launch, beyond through the full
+    // planes (the plane buffer of the Fourier-plane requests, batch-sized)
     if ((mode == 0 && ((1 << fp.logW) >= 256 || !isPow2(fp.w) || !isPow2(fp.h))) || mode == 5) {
+        fe = dh_launch_forward_win(fp, o.stream);
+        if (fe == cudaSuccess) { o.lastForwardKernel = 5; return fe; }
+        if (fe != cudaErrorNotSupported) return fe;
+        cudaGetLastError();
         const size_t Nx = (size_t)(1 << fp.logW) / 2 + 1;
         const size_t frames = (size_t)std::max(o.batchCount * std::max(1, o.avgCount), fp.frameOffset + fp.frameCount);
         const size_t need = frames * o.polCount * (1 << fp.logH) * Nx * sizeof(float2);
