@@ -335,7 +335,7 @@ __global__ void __launch_bounds__(NT, 1)
     const int yr = ref[2 * N + y], yi = ref[3 * N + y];
     const float yv = p.yAxis[y];
     const float yw = yv + (yv < 0.f ? fabsf((p.yAxis[1] - p.yAxis[0]) * (float)N) : 0.f);
-    const float x0 = p.xAxis[0], dx = p.xAxis[1] - x0;
+    const float dx = p.xAxis[1] - p.xAxis[0], xc = p.xAxis[N / 2];
     const float inv = 1.0f / (float)(N * N);
     unsigned char* myStg = stg + y * 128 + 2 * u;
     const int sw = (y & 7) << 4;
@@ -516,15 +516,15 @@ __global__ void __launch_bounds__(NT, 1)
             mx = fmaxf(fmaxf(mx, v.x), v.y);
             const f2x I = mul2(I0, inv2);
             sP = add2(sP, I);
-            sX = fma2(I, pk1((float)(8 * brev4c(i))), sX);
+            sX = fma2(I, pk1((float)(8 * brev4c(i) - N / 2)), sX);
             sE = fma2(I, I, sE);
         }
         {
             const float2 v = upk(sP), t = upk(sX), e = upk(sE);
             const float Prow = v.x + v.y;
-            const float xs = fmaf((float)u, Prow, v.y) + (t.x + t.y);   // sum of I x / dx
+            const float xs = fmaf((float)u, Prow, v.y) + (t.x + t.y);   // x = dx (index - N / 2) + xc
             red[tid] = Prow;
-            red[NT + tid] = fmaf(dx, xs, x0 * Prow);
+            red[NT + tid] = fmaf(dx, xs, xc * Prow);
             red[2 * NT + tid] = yv * Prow;
             red[3 * NT + tid] = yw * Prow;
             red[4 * NT + tid] = e.x + e.y;

@@ -28,8 +28,8 @@ cudaError_t dh_launch_forward_i8(const DhFwdParams& p, cudaStream_t s);
 cudaError_t dh_launch_forward_i8_fused(const DhFwdParams& p, const DhInvParams& ip, cudaStream_t s);
 cudaError_t dh_launch_fourier_full(const DhFourierParams& q, cudaStream_t s);
 cudaError_t dh_launch_forward_plane(const DhFourierParams& q, cudaStream_t s);
-size_t dh_field_band64_scratch_bytes(const DhInvParams& p, int overlapKind);
-cudaError_t dh_launch_field_band64(const DhInvParams& p, int overlapKind, void* scratch, size_t scratchBytes,
+size_t dh_field512_scratch_bytes(const DhInvParams& p, int overlapKind);
+cudaError_t dh_launch_field512(const DhInvParams& p, int overlapKind, void* scratch, size_t scratchBytes,
                                    int* overlapUsed, cudaStream_t s);
 int dh_forward_i8_npad(int w);
 cudaError_t dh_launch_inverse_lo(const DhInvParams& p, cudaStream_t s);
@@ -859,8 +859,8 @@ static cudaError_t launchBands(Object& o, const DhInvParams& ip, bool mayAlloc) 
         return e;
     }
     // 512-wide fields with IFFT windows up to 64 x 64: 64-point sub-transforms
-    // and the exact integer overlap (dh_band64.cu)
-    const size_t need64 = dh_field_band64_scratch_bytes(ip, o.overlapKernel);
+    // and the exact integer overlap (dh_field512.cu)
+    const size_t need64 = dh_field512_scratch_bytes(ip, o.overlapKernel);
     if (need64 > 0) {
         if (o.dBigScratch.bytes < need64) {
             if (!mayAlloc) return cudaErrorMemoryAllocation;
@@ -868,7 +868,7 @@ static cudaError_t launchBands(Object& o, const DhInvParams& ip, bool mayAlloc) 
             if (e != cudaSuccess) return e;
         }
         int used = 0;
-        cudaError_t e = dh_launch_field_band64(ip, o.overlapKernel, o.dBigScratch.ptr, o.dBigScratch.bytes, &used, o.stream);
+        cudaError_t e = dh_launch_field512(ip, o.overlapKernel, o.dBigScratch.ptr, o.dBigScratch.bytes, &used, o.stream);
         if (e == cudaSuccess) {
             o.lastInverseKernel = 7;
             o.lastOverlapKernel = used;

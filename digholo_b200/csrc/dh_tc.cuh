@@ -122,6 +122,16 @@ __device__ __forceinline__ void tmemWaitLoad8(uint32_t (&r)[8]) {
                  : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])::"memory");
 }
 
+// The same for 4 columns.
+__device__ __forceinline__ void tmemLoad4(uint32_t taddr, uint32_t (&r)[4]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(taddr));
+}
+__device__ __forceinline__ void tmemWaitLoad4(uint32_t (&r)[4]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3])::"memory");
+}
+
 // Exact split of 8 int16 values into bf16 hi and lo (element order kept).
 __device__ __forceinline__ void split8(const uint4 raw, uint4& hi, uint4& lo) {
     const unsigned w[4] = {raw.x, raw.y, raw.z, raw.w};
