@@ -26,6 +26,7 @@
 #include <stdint.h>
 
 #include "dh_common.cuh"
+#include "dh_f32x2.cuh"
 #include "dh_grad.h"
 #include "dh_host.h"
 
@@ -268,6 +269,169 @@ __global__ void __launch_bounds__(256) k_align_grad_reg(DhGradParams p) {
     }
 }
 
+// The same contraction with four columns per thread in packed pairs (f32x2),
+// G <= GM - 2: lanes along the columns, four each, so that one shared load
+// serves four pixels and one instruction two.  The waist derivative's adjoint
+// field is written in the modes themselves, the ladder relation applied to
+// the coefficients instead of the modes:
+//   Abar_w = sum_mn D_mn Hx_m Hy_n,  D_mn = -(1 / 2w) (
+//       sqrt((m+1)(m+2)) conj(c_{m+2,n}) - sqrt((m-1) m) conj(c_{m-2,n}) + (same in n)),
+// m + n < G + 2, which leaves four FMAs per pixel and mode where the
+// derivative modes need six.  Bound: latency (32 % of the issue slots at 16
+// warps per SM; 2.9 TB/s of V, Vx, Vy).  1024 fields of 128 x 128, 15 groups:
+// 141 us; k_align_grad_reg 195.
+template <int GM, int CP>
+__global__ void __launch_bounds__(256) k_align_grad_tile(DhGradParams p) {
+    extern __shared__ float4 sg4[];
+    const int unit = blockIdx.x;
+    const int P = p.polCount, G = p.G, M = p.M, nx = p.nx, ny = p.ny;
+    const int pol = unit % P, frame = unit / P;
+    const int GE = G + 2;
+    float4* UD = sg4;                                                 // [ny][GM][2] {ux, ux, uy, uy}, {dx, dx, dy, dy}
+    float4* CD = UD + (size_t)2 * GM * ny;                            // [n][m] {conj(c), D}
+    float* red = reinterpret_cast<float*>(CD + GM * GM);              // [8 warps][7]
+    const float* hxp = p.hx + (size_t)pol * GE * nx;
+    const float* hyp = p.hy + (size_t)pol * GE * ny;
+    const float ladder = -1.0f / (2.0f * p.waist[pol]);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+
+    float spow = 0.f;
+    for (int mode = tid; mode < M; mode += blockDim.x) {
+        const float2 c = p.coefs[(size_t)frame * P * M + (size_t)pol * M + mode];
+        spow = fmaf(c.x, c.x, fmaf(c.y, c.y, spow));
+    }
+    const float2* src = (p.weights ? p.weights : p.coefs) + (size_t)frame * P * M + (size_t)pol * M;
+    const float sgn = p.weights ? 1.0f : -1.0f;
+    auto coef = [&](int m, int n) {
+        if (m < 0 || n < 0 || m + n >= G) return make_float2(0.f, 0.f);
+        const int g = m + n;
+        const float2 c = src[g * (g + 1) / 2 + n];
+        return make_float2(c.x, sgn * c.y);
+    };
+    for (int e = tid; e < GM * GM; e += 256) {
+        const int n = e / GM, m = e - n * GM;
+        const float2 c = coef(m, n), a = coef(m + 2, n), b = coef(m - 2, n), d = coef(m, n + 2), f = coef(m, n - 2);
+        const float wa = sqrtf((float)((m + 1) * (m + 2))), wb = sqrtf((float)((m - 1) * m));
+        const float wd = sqrtf((float)((n + 1) * (n + 2))), wf = sqrtf((float)((n - 1) * n));
+        CD[e] = make_float4(c.x, c.y, ladder * (wa * a.x - wb * b.x + wd * d.x - wf * f.x),
+                            ladder * (wa * a.y - wb * b.y + wd * d.y - wf * f.y));
+    }
+    __syncthreads();
+    // row sums: each thread one y, every second m
+    for (int y = tid >> 1; y < ny; y += 128) {
+        constexpr int HM = GM / 2;
+        const int par = tid & 1;
+        f2x us[HM], ds[HM];
+#pragma unroll
+        for (int i = 0; i < HM; i++) us[i] = ds[i] = pk(0.f, 0.f);
+        for (int n = 0; n < GE; n++) {
+            const f2x h = pk1(__ldg(hyp + (size_t)n * ny + y));
+            const ulonglong2* c = reinterpret_cast<const ulonglong2*>(CD + n * GM + par);
+#pragma unroll
+            for (int i = 0; i < HM; i++) {
+                const ulonglong2 v = c[2 * i];
+                us[i] = fma2(v.x, h, us[i]);
+                ds[i] = fma2(v.y, h, ds[i]);
+            }
+        }
+        float4* o = UD + ((size_t)y * GM + par) * 2;
+#pragma unroll
+        for (int i = 0; i < HM; i++) {
+            const float2 u = upk(us[i]), d = upk(ds[i]);
+            o[4 * i] = make_float4(u.x, u.x, u.y, u.y);
+            o[4 * i + 1] = make_float4(d.x, d.x, d.y, d.y);
+        }
+    }
+    __syncthreads();
+
+    const size_t base = (size_t)unit * nx * ny;
+    constexpr int CT = 2 * CP;                       // columns per thread
+    const int LX = nx / CT < 32 ? nx / CT : 32;      // lanes per row (nx is a power of two, at least CT)
+    const int rows = 8 * (32 / LX);                  // rows in flight per block
+    const int y0 = warp * (32 / LX) + lane / LX;
+    const float bx = p.bcx[pol], by = p.bcy[pol];
+    // sums: Im(Abar V) (x + bcx), Im(Abar V) (y + bcy), Im(Abar V) (x^2 + y^2),
+    // Re(Abar Vx), Re(Abar Vy), Re(Abar_w V), Im(Abar V)
+    float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f, s4 = 0.f, s5 = 0.f, si = 0.f;
+    for (int x0 = (lane % LX) * CT; x0 < nx; x0 += LX * CT) {
+        f2x hr[CP][GM];
+#pragma unroll
+        for (int q = 0; q < CP; q++)
+#pragma unroll
+            for (int m = 0; m < GM; m++) {
+                const float2 v = m < GE ? __ldg(reinterpret_cast<const float2*>(hxp + (size_t)m * nx + x0 + 2 * q)) : make_float2(0.f, 0.f);
+                hr[q][m] = pk(v.x, v.y);
+            }
+        float col[CT];
+#pragma unroll
+        for (int q = 0; q < CT; q++) col[q] = 0.f;
+        for (int y = y0; y < ny; y += rows) {
+            const size_t e = base + (size_t)y * nx + x0;
+            float4 v[CP], vx[CP], vy[CP];
+#pragma unroll
+            for (int q = 0; q < CP; q++) {
+                v[q] = __ldg(reinterpret_cast<const float4*>(p.V + e) + q);
+                vx[q] = __ldg(reinterpret_cast<const float4*>(p.Vx + e) + q);
+                vy[q] = __ldg(reinterpret_cast<const float4*>(p.Vy + e) + q);
+            }
+            f2x ar[CP], ai[CP], wr[CP], wi[CP];
+#pragma unroll
+            for (int q = 0; q < CP; q++) ar[q] = ai[q] = wr[q] = wi[q] = pk(0.f, 0.f);
+            const ulonglong2* u = reinterpret_cast<const ulonglong2*>(UD + (size_t)y * GM * 2);
+#pragma unroll
+            for (int m = 0; m < GM; m++) {
+                const ulonglong2 uc = u[2 * m], dc = u[2 * m + 1];
+#pragma unroll
+                for (int q = 0; q < CP; q++) {
+                    if (m < GM - 2) {
+                        ar[q] = fma2(hr[q][m], uc.x, ar[q]);
+                        ai[q] = fma2(hr[q][m], uc.y, ai[q]);
+                    }
+                    wr[q] = fma2(hr[q][m], dc.x, wr[q]);
+                    wi[q] = fma2(hr[q][m], dc.y, wi[q]);
+                }
+            }
+            float row = 0.f;
+#pragma unroll
+            for (int q = 0; q < CP; q++) {
+                const float2 axr = upk(ar[q]), axi = upk(ai[q]), awr = upk(wr[q]), awi = upk(wi[q]);
+                const float im0 = axr.x * v[q].y + axi.x * v[q].x, im1 = axr.y * v[q].w + axi.y * v[q].z;
+                col[2 * q] += im0;
+                col[2 * q + 1] += im1;
+                row += im0 + im1;
+                s3 += (axr.x * vx[q].x - axi.x * vx[q].y) + (axr.y * vx[q].z - axi.y * vx[q].w);
+                s4 += (axr.x * vy[q].x - axi.x * vy[q].y) + (axr.y * vy[q].z - axi.y * vy[q].w);
+                s5 += (awr.x * v[q].x - awi.x * v[q].y) + (awr.y * v[q].z - awi.y * v[q].w);
+            }
+            const float yv = p.yAxis[y];
+            s1 = fmaf(row, yv + by, s1);
+            s2 = fmaf(row, yv * yv, s2);
+        }
+#pragma unroll
+        for (int q = 0; q < CT; q++) {
+            const float xv = p.xAxis[x0 + q];
+            s0 = fmaf(col[q], xv + bx, s0);
+            s2 = fmaf(col[q], xv * xv, s2);
+            si += col[q];
+        }
+    }
+    const float k0u = p.k0u[pol];
+    // Re(Abar V i) = -Im(Abar V); the beam-centre tangents carry -Im(Abar V) k0 u t
+    float s[7] = {-k0u * s0, -k0u * s1, -p.piOverLambda * s2, s3 - k0u * p.tiltX[pol] * si,
+                  s4 - k0u * p.tiltY[pol] * si, s5, spow};
+#pragma unroll
+    for (int k = 0; k < 7; k++)
+        for (int off = 16; off > 0; off >>= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], off);
+    if (lane == 0)
+        for (int k = 0; k < 7; k++) red[warp * 7 + k] = s[k];
+    __syncthreads();
+    if (tid < 7) {
+        float t = 0.f;
+        for (int wv = 0; wv < 8; wv++) t += red[wv * 7 + tid];
+        p.out[(size_t)unit * 7 + tid] = t;
+    }
+}
+
 // The power term of the gradient kernels alone (their first loop and their
 // block reduction, in the same order).
 __global__ void __launch_bounds__(256) k_align_power(DhGradParams p) {
@@ -369,8 +533,28 @@ static cudaError_t launchAlignGradReg(const DhGradParams& p, size_t smem, cudaSt
     return cudaGetLastError();
 }
 
+template <int GM, int CP>
+static cudaError_t launchAlignGradTile(const DhGradParams& p, cudaStream_t s) {
+    const size_t smem = sizeof(float4) * ((size_t)2 * GM * p.ny + GM * GM) + sizeof(float) * 8 * 7;
+    if (smem > 200 * 1024) return cudaErrorNotSupported;
+    cudaError_t e = setSmemOnce(reinterpret_cast<const void*>(k_align_grad_tile<GM, CP>), (int)smem);
+    if (e != cudaSuccess) return e;
+    k_align_grad_tile<GM, CP><<<(unsigned)(p.frameCount * p.polCount), 256, smem, s>>>(p);
+    return cudaGetLastError();
+}
+
 cudaError_t dh_launch_align_grad(const DhGradParams& p, cudaStream_t s) {
     const bool pow2 = p.nx > 0 && (p.nx & (p.nx - 1)) == 0;
+    // four (G <= 16) or two columns per thread where the row sums fit shared
+    // memory (18 or 34 modes x 32 bytes x ny: up to 256 and 128 rows), else
+    // one column per thread
+    if (pow2 && p.nx >= 16 && p.G <= 32 &&
+        ((reinterpret_cast<uintptr_t>(p.V) | reinterpret_cast<uintptr_t>(p.Vx) | reinterpret_cast<uintptr_t>(p.Vy)) & 15) == 0 &&
+        (reinterpret_cast<uintptr_t>(p.hx) & 7) == 0) {
+        const cudaError_t e = p.G <= 16 ? launchAlignGradTile<18, 2>(p, s) : launchAlignGradTile<34, 1>(p, s);
+        if (e != cudaErrorNotSupported) return e;
+        cudaGetLastError();
+    }
     if (pow2 && p.G <= 32) {
         const int GM = p.G <= 16 ? 16 : 32;
         const size_t smemReg = sizeof(float4) * (size_t)GM * p.ny + sizeof(float2) * (size_t)p.M +
