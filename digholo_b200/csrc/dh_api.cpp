@@ -80,6 +80,7 @@ int digHoloDestroy(int h) {
             if (o->d2hStream) cudaStreamDestroy(o->d2hStream);
             for (auto e : o->evChunk) if (e) cudaEventDestroy(e);
             if (o->evD2H) cudaEventDestroy(o->evD2H);
+            if (o->evMetric) cudaEventDestroy(o->evMetric);
             if (o->evStart) cudaEventDestroy(o->evStart);
             if (o->evStop) cudaEventDestroy(o->evStop);
             if (o->hStatus) cudaFreeHost(o->hStatus);

@@ -12,6 +12,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <memory>
 #include <vector>
 
 #include "dh_object.h"
@@ -44,30 +45,21 @@ struct Block {
     int pol0, pol1, rows;
 };
 
-// The smallest and largest squared singular value of a block and the sum of
-// all of them (its squared Frobenius norm), via the extreme eigenvalues and
-// the trace of its smaller Gram matrix.
-static int blockSingular2(Object& o, const Block& blk, double& s2min, double& s2max, double& s2sum) {
+// Enqueues the smallest and largest squared singular value of a block and the
+// sum of all of them (its squared Frobenius norm), via the extreme eigenvalues
+// and the trace of its smaller Gram matrix: W[0], W[n - 1], W[n] on the device.
+static int launchSingular2(Object& o, const Block& blk, double* W) {
     const int B = o.batchCount, M = objOutputModes(o), P = o.polCount;
     const size_t aBytes = (size_t)blk.rows * B * sizeof(float2);
     const int rowsGram = blk.rows <= B;
     const int n = rowsGram ? blk.rows : B;
     if (o.dMetricA.ensure(aBytes) != cudaSuccess) return ERR_MEMORYALLOCATION;
-    if (o.dMetricG.ensure((size_t)n * n * 16 + (size_t)(n + 1) * sizeof(double)) != cudaSuccess) return ERR_MEMORYALLOCATION;
+    if (o.dMetricG.ensure((size_t)n * n * 16) != cudaSuccess) return ERR_MEMORYALLOCATION;
     if (dh_launch_gather_block(blk.src0, blk.src1, blk.pol0, blk.pol1, P, M, blk.rows, B, o.dMetricA.as<float2>(),
                                o.stream) != cudaSuccess) return ERR_ERROR;
     if (dh_launch_gram(o.dMetricA.as<float2>(), blk.rows, B, rowsGram, o.dMetricG.ptr, o.stream) != cudaSuccess) return ERR_ERROR;
-    double* W = reinterpret_cast<double*>(o.dMetricG.as<char>() + (size_t)n * n * 16);   // [n] + trace
     if (!o.eigen) o.eigen = dh_eigen_create();
     if (dh_eigen_extremes(*o.eigen, o.dMetricG.ptr, n, 1, W, nullptr, W + n, o.stream)) return ERR_ERROR;
-    double h[3];
-    if (cudaMemcpyAsync(&h[0], W, sizeof(double), cudaMemcpyDeviceToHost, o.stream) != cudaSuccess ||
-        cudaMemcpyAsync(&h[1], W + n - 1, 2 * sizeof(double), cudaMemcpyDeviceToHost, o.stream) != cudaSuccess)
-        return ERR_ERROR;
-    if (cudaStreamSynchronize(o.stream) != cudaSuccess) return ERR_ERROR;
-    s2min = h[0] < 0 ? 0 : h[0];
-    s2max = h[1] < 0 ? 0 : h[1];
-    s2sum = h[2] < 0 ? 0 : h[2];
     return ERR_SUCCESS;
 }
 
@@ -144,18 +136,52 @@ int powerMeter(Object& o, float* out, int polIdx, int polsIndependent, const flo
     float il = 0.f, mdl = 0.f;
     for (int i = 0; i < METRIC_COUNT; i++) out[i] = 0.f;
     if (M <= 0 || !coefs) return ERR_NULLPOINTER;
-    // host copy of the coefficients for the element-wise metrics
-    std::vector<float> hc((size_t)B * P * M * 2);
-    if (cudaMemcpyAsync(hc.data(), coefs, hc.size() * sizeof(float), cudaMemcpyDeviceToHost, o.stream) != cudaSuccess)
-        return ERR_ERROR;
-    std::vector<float> ho;
     const float2* otherSrc = other ? other : coefs;
+    // matrix blocks (digHolo.cpp:10771-10912), each element (row j, batch b)
+    const bool indep = polsIndependent || P == 1;
+    std::vector<Block> blocks;
+    if (P == 1) {
+        blocks.push_back({coefs, coefs, 0, 0, M});
+    } else if (polIdx >= 0) {
+        if (indep) blocks.push_back({coefs, coefs, polIdx, polIdx, M});
+        else blocks.push_back({coefs, otherSrc, polIdx, 1 - polIdx, 2 * M});
+    } else {
+        if (indep) {
+            blocks.push_back({coefs, coefs, 0, 0, M});
+            blocks.push_back({coefs, coefs, 1, 1, M});
+        } else {
+            blocks.push_back({coefs, coefs, 0, 1, 2 * M});
+        }
+    }
+    const int svdM = blocks[0].rows;
+    const int svdN = B;
+    const int svdCount = (int)blocks.size();
+    // IL and MDL on the device, enqueued first: the copy and the element-wise
+    // metrics below run while the eigen solver does (the coefficients are
+    // complete at evMetric, and the copy is waited for before this returns)
+    const int minDim = std::min(svdM, svdN);
+    const bool svd = doMDL && B > 1;
+    if (cudaEventRecord(o.evMetric, o.stream) != cudaSuccess) return ERR_ERROR;
+    if (svd) {
+        if (o.dMetricW.ensure((size_t)svdCount * (minDim + 1) * sizeof(double)) != cudaSuccess) return ERR_MEMORYALLOCATION;
+        for (int k = 0; k < svdCount; k++) {
+            const int r = launchSingular2(o, blocks[k], o.dMetricW.as<double>() + (size_t)k * (minDim + 1));
+            if (r) return r;
+        }
+    }
+
+    // host copy of the coefficients for the element-wise metrics
+    const size_t elems = (size_t)B * P * M * 2;
+    std::unique_ptr<float[]> hc(new float[elems]), ho;
+    if (cudaStreamWaitEvent(o.d2hStream, o.evMetric, 0) != cudaSuccess ||
+        cudaMemcpyAsync(hc.get(), coefs, elems * sizeof(float), cudaMemcpyDeviceToHost, o.d2hStream) != cudaSuccess)
+        return ERR_ERROR;
     if (P == 2 && polIdx >= 0 && !polsIndependent) {
-        ho.resize(hc.size());
-        if (cudaMemcpyAsync(ho.data(), otherSrc, ho.size() * sizeof(float), cudaMemcpyDeviceToHost, o.stream) != cudaSuccess)
+        ho.reset(new float[elems]);
+        if (cudaMemcpyAsync(ho.get(), otherSrc, elems * sizeof(float), cudaMemcpyDeviceToHost, o.d2hStream) != cudaSuccess)
             return ERR_ERROR;
     }
-    if (cudaStreamSynchronize(o.stream) != cudaSuccess) return ERR_ERROR;
+    if (cudaStreamSynchronize(o.d2hStream) != cudaSuccess) return ERR_ERROR;
 
     if (B <= 1) {  // digHolo.cpp:11078-11111
         float total = 0.f, diag = 0.f;
@@ -178,44 +204,25 @@ int powerMeter(Object& o, float* out, int polIdx, int polsIndependent, const flo
         return ERR_SUCCESS;
     }
 
-    // matrix blocks (digHolo.cpp:10771-10912), each element (row j, batch b)
-    const bool indep = polsIndependent || P == 1;
-    std::vector<Block> blocks;
-    int svdM = 0;
     // host view: element(j, b) of block k
     auto hostElem = [&](int k, int j, int b, float& re, float& im) {
         const Block& bl = blocks[k];
         const int Mx = M;
         const float* src;
         int pol, jj;
-        if (j < Mx) { src = (bl.src0 == coefs) ? hc.data() : ho.data(); pol = bl.pol0; jj = j; }
-        else { src = (bl.src1 == coefs) ? hc.data() : ho.data(); pol = bl.pol1; jj = j - Mx; }
+        if (j < Mx) { src = (bl.src0 == coefs) ? hc.get() : ho.get(); pol = bl.pol0; jj = j; }
+        else { src = (bl.src1 == coefs) ? hc.get() : ho.get(); pol = bl.pol1; jj = j - Mx; }
         const size_t i = ((size_t)b * P * Mx + (size_t)pol * Mx + jj) * 2;
         re = src[i];
         im = src[i + 1];
     };
-    if (P == 1) {
-        blocks.push_back({coefs, coefs, 0, 0, M});
-    } else if (polIdx >= 0) {
-        if (indep) blocks.push_back({coefs, coefs, polIdx, polIdx, M});
-        else blocks.push_back({coefs, otherSrc, polIdx, 1 - polIdx, 2 * M});
-    } else {
-        if (indep) {
-            blocks.push_back({coefs, coefs, 0, 0, M});
-            blocks.push_back({coefs, coefs, 1, 1, M});
-        } else {
-            blocks.push_back({coefs, coefs, 0, 1, 2 * M});
-        }
-    }
-    svdM = blocks[0].rows;
-    const int svdN = B;
-    const int svdCount = (int)blocks.size();
-
     float totalSignal = 0, totalNoise = 0, totalSNR = 0, totalSignalMG = 0, totalNoiseMG = 0;
     float minSignal = FLT_MAX, maxSignal = -FLT_MAX, minNoise = FLT_MAX, maxNoise = -FLT_MAX;
     float minSNR = FLT_MAX, maxSNR = -FLT_MAX;
     int totalSignalCount = 1;
     if (doXtalk) {  // digHolo.cpp:10924-11008
+        std::vector<int> group(M);
+        for (int m = 0; m < M; m++) group[m] = hgGroup(m) + 1;
         for (int k = 0; k < svdCount; k++) {
             int Mv = svdM, Nv = svdN;
             std::vector<double> uu;
@@ -241,9 +248,9 @@ int powerMeter(Object& o, float* out, int polIdx, int polsIndependent, const flo
             totalSignalCount = Mv * Nv * svdCount;
             for (int i = 0; i < Nv && i < M; i++) {
                 float signal = 0, noise = 0;
-                const int MGin = hgGroup(i) + 1;
+                const int MGin = group[i];
                 for (int j = 0; j < Mv; j++) {
-                    const int MGout = hgGroup(j % M) + 1;
+                    const int MGout = group[j % M];
                     float vr, vi;
                     if (!uu.empty()) {
                         // column-major n x n: element (j, i) at i * n + j
@@ -276,16 +283,18 @@ int powerMeter(Object& o, float* out, int polIdx, int polsIndependent, const flo
     if (doMDL) {  // digHolo.cpp:11012-11062
         // IL: the mean squared singular value (the trace of the Gram matrix
         // over its size); MDL: the smallest over the largest, over all blocks
-        const int minDim = std::min(svdM, svdN);
         double sum = 0.0;
         float maxS = -FLT_MAX, minS = FLT_MAX;
+        std::vector<double> ev((size_t)svdCount * (minDim + 1));
+        if (cudaMemcpyAsync(ev.data(), o.dMetricW.ptr, ev.size() * sizeof(double), cudaMemcpyDeviceToHost, o.stream) != cudaSuccess ||
+            cudaStreamSynchronize(o.stream) != cudaSuccess)
+            return ERR_ERROR;
         for (int k = 0; k < svdCount; k++) {
-            double lo2 = 0.0, hi2 = 0.0, sum2 = 0.0;
-            const int r = blockSingular2(o, blocks[k], lo2, hi2, sum2);
-            if (r) return r;
-            sum += sum2;
-            minS = std::min(minS, (float)std::sqrt(lo2));
-            maxS = std::max(maxS, (float)std::sqrt(hi2));
+            const double* e = ev.data() + (size_t)k * (minDim + 1);
+            auto positive = [](double v) { return v < 0 ? 0 : v; };
+            sum += positive(e[minDim]);
+            minS = std::min(minS, (float)std::sqrt(positive(e[0])));
+            maxS = std::max(maxS, (float)std::sqrt(positive(e[minDim - 1])));
         }
         il = (float)(sum / ((double)svdCount * minDim));
         mdl = (minS * minS) / (maxS * maxS);

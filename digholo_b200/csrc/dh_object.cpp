@@ -283,6 +283,7 @@ int objInitDevice(Object& o) {
     DH_CUDA(o, cudaEventCreateWithFlags(&o.evChunk[0], cudaEventDisableTiming));
     DH_CUDA(o, cudaEventCreateWithFlags(&o.evChunk[1], cudaEventDisableTiming));
     DH_CUDA(o, cudaEventCreateWithFlags(&o.evD2H, cudaEventDisableTiming));
+    DH_CUDA(o, cudaEventCreateWithFlags(&o.evMetric, cudaEventDisableTiming));
     DH_CUDA(o, cudaEventCreate(&o.evStart));
     DH_CUDA(o, cudaEventCreate(&o.evStop));
     // twiddle(k) = exp(-2 pi i k / 4096), double precision rounded to float

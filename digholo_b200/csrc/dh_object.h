@@ -137,6 +137,7 @@ struct Object {
     cudaStream_t d2hStream = nullptr;
     cudaEvent_t evChunk[2] = {nullptr, nullptr};
     cudaEvent_t evD2H = nullptr;
+    cudaEvent_t evMetric = nullptr;   // the coefficients a power meter reads are complete
     cudaEvent_t evStart = nullptr, evStop = nullptr;
     int userStream = 0;                 // stream supplied by digHoloB200SetStream (not owned)
     int timing = 0;                     // record per-stage events in ProcessBatch
@@ -175,7 +176,7 @@ struct Object {
     int basisPolCount = 0;
     int keepField32 = 0;
     // power meter / AutoAlign
-    DevBuf dMetricA, dMetricG, dCoefsBackup, dAlignFrames;
+    DevBuf dMetricA, dMetricG, dMetricW, dCoefsBackup, dAlignFrames;
     DevBuf dDigits;                     // tensor-core row DFT digits (uint16 frames)
     // Fourier planes of the last batch (on request): the frame source the
     // batch was processed from, the planes, their statistics and batch sum
