@@ -94,6 +94,7 @@ constexpr int RN = 256;          // complex points per row (W = 512)
 
 constexpr int NG = 4;            // row groups per block, the next one's pixels prefetched into registers
 
+
 // Loads of row group g (16 rows of one unit): 16-byte loads, 8 uint16 or 4
 // float pixels each, into registers.
 template <bool U16>
@@ -133,11 +134,17 @@ struct RowRaw {
 // compact = 0: the plane's layout ([unit][H][W/2 + 1]).  A block takes NG
 // consecutive groups of 16 rows.  A row's 16 threads are 16 lanes of one
 // warp, so its exchange needs only warp barriers; the exchange reuses the
-// row's buffer, value (k1, t) at 16 k1 + (t ^ k1).
+// row's buffer, value (k1, t) at 16 k1 + (t ^ k1).  The twiddles sit in shared
+// memory, by (k1, t): from the global table, whose entries for neighbouring
+// lanes are 128 bytes apart, they cost 16 L1 wavefronts a load and twice the
+// kernel's time (96 x 2 windows of uint16: 147 us; 75 with the shared table, at
+// 71 % of the issue slots, which bound it now; persistent blocks: the same).
 template <bool U16>
 __global__ void __launch_bounds__(256, U16 ? 4 : 3) k_plane_rows512(DhFourierParams q, int compact) {
     extern __shared__ float2 sp[];
     float2* A = sp;                          // [RR][RN] z, the exchange, then X
+    float2* tw = A + RR * RN;                // [16 k1][16 t]: exp(-2 pi i t k1 / 256)
+    float2* ws = tw + RN;                    // exp(-2 pi i k / 512) of the kept columns
     const DhFwdParams& f = q.f;
     const int H = 1 << f.logH, Nx = RN + 1;
     const int groups = H / RR;
@@ -148,6 +155,8 @@ __global__ void __launch_bounds__(256, U16 ? 4 : 3) k_plane_rows512(DhFourierPar
     float2* Ar = A + r * RN;
     RowRaw<U16> raw;
     raw.load(f, g0 / groups, (g0 % groups) * RR, tid);
+    tw[tid] = __ldg(&f.twiddle[(t * r) << (TW_LOG - 8)]);
+    for (int k = tid; k < Nx; k += 256) ws[k] = __ldg(&f.twiddle[k << (TW_LOG - 9)]);
     for (int gi = 0; gi < NG; gi++) {
         const int g = g0 + gi;
         if (g >= total) break;
@@ -166,7 +175,7 @@ __global__ void __launch_bounds__(256, U16 ? 4 : 3) k_plane_rows512(DhFourierPar
 #pragma unroll
         for (int k1 = 0; k1 < 16; k1++) {
             float2 y = at16(v, k1);
-            if (k1 && t) y = cmul(y, __ldg(&f.twiddle[(t * k1) << (TW_LOG - 8)]));
+            if (k1 && t) y = cmul(y, tw[16 * k1 + t]);
             Ar[16 * k1 + (t ^ k1)] = y;
         }
         __syncwarp();
@@ -190,7 +199,7 @@ __global__ void __launch_bounds__(256, U16 ? 4 : 3) k_plane_rows512(DhFourierPar
             const float2 even = cscale(cadd(zk, zc), 0.5f);
             const float2 d = csub(zk, zc);
             const float2 odd = make_float2(0.5f * d.y, -0.5f * d.x);
-            const float2 wk = __ldg(&f.twiddle[k << (TW_LOG - 9)]);
+            const float2 wk = ws[k];
             out[(size_t)rr * pitch + (k - o0)] = cadd(even, cmul(wk, odd));
         }
     }
@@ -203,13 +212,17 @@ namespace {
 
 constexpr int WC = 8;            // window columns per block
 constexpr int WT = 512;          // threads per block
-constexpr int WEX = 65;          // padded stride of the exchange and of Z
+constexpr int WEX = 65;          // padded stride of the exchange
+constexpr int WZ = 66;           // and of Z: eight columns and two rows of a half-warp in distinct banks
 
 // One block: WC columns c0 .. c0 + 7 of one (frame, polarisation), from the
 // compact row output ([unit][H][w]).  H = 64 Q rows, Q <= 8, so the
 // WC Q <= 64 decimated transforms take one pass of 64 x 8 threads: thread
-// (a2, s) with s = tid mod 64 the transform (column s / Q, sequence s mod Q)
-// and a2 = tid / 64 its slot.
+// (a2, s) with s = tid mod 64 the transform (column s mod 8, sequence s / 8)
+// and a2 = tid / 64 its slot.  The last stage has the eight columns on
+// neighbouring lanes, so that the factors and the window move in runs of 64
+// bytes (192 units, H = 512: 50 us with neighbouring rows there, 34 so, at
+// half of the issue slots).  Bound: the shared-memory exchanges.
 __global__ void __launch_bounds__(WT) k_plane_window64(DhFourierParams q) {
     extern __shared__ float2 sw[];
     const DhFwdParams& f = q.f;
@@ -218,9 +231,9 @@ __global__ void __launch_bounds__(WT) k_plane_window64(DhFourierParams q) {
     const int cgroups = w / WC;
     const int unit = blockIdx.x / cgroups, c0 = (blockIdx.x % cgroups) * WC;
     const int pol = unit % P, frame = unit / P;
-    const int HS = H + 8;                       // padded column stride of S
-    float2* S = sw;                             // [WC][HS]: the columns, then Z [s][WEX]
-    float2* Ex = sw + WC * HS;                  // [8 k1][8 a2][WEX]
+    const int HS = H + 2;                       // padded column stride of S
+    float2* S = sw;                             // [WC][HS]: the columns, then Z [s][WZ]
+    float2* Ex = sw + WC * max(HS, Q * WZ);     // [8 k1][8 a2][WEX]
     const int tid = threadIdx.x;
     const float2* pl = q.plane + (size_t)unit * H * w + c0;
     // columns in: 8 consecutive complex values (64 bytes) of each row
@@ -235,7 +248,7 @@ __global__ void __launch_bounds__(WT) k_plane_window64(DhFourierParams q) {
     const int NS = WC * Q;
     const int s = tid & 63, a2 = tid >> 6;
     const bool act = s < NS;
-    const int c = act ? s / Q : 0, b = act ? s - (s / Q) * Q : 0;
+    const int c = s & (WC - 1), b = act ? s / WC : 0;
     float2 v[8];
 #pragma unroll
     for (int a1 = 0; a1 < 8; a1++) v[a1] = act ? S[c * HS + Q * (8 * a1 + a2) + b] : make_float2(0.f, 0.f);
@@ -255,7 +268,7 @@ __global__ void __launch_bounds__(WT) k_plane_window64(DhFourierParams q) {
     float2* Z = S;
     if (act) {
 #pragma unroll
-        for (int k2 = 0; k2 < 8; k2++) Z[s * WEX + a2 + 8 * k2] = v[k2];
+        for (int k2 = 0; k2 < 8; k2++) Z[s * WZ + a2 + 8 * k2] = v[k2];
     }
     __syncthreads();
     // the kept rows j: X[row_j] = sum_b exp(-2 pi i row_j b / H) Z_b[row_j mod 64],
@@ -264,12 +277,12 @@ __global__ void __launch_bounds__(WT) k_plane_window64(DhFourierParams q) {
     if (f.batchCal && f.batchCalCount > 0)
         bc = f.batchCal[pol * f.batchCalCount + ((f.frameOffset + frame) % f.batchCalCount)];
     {
-        const int j = tid & 63, cc = tid >> 6;   // 64 rows x 8 columns
+        const int j = tid >> 3, cc = tid & 7;    // 64 rows x 8 columns
         const int row = ((j + f.sy[pol] + H / 2) % H + H) % H;
         const int m = row & 63;
         const float2* tc = f.tabCol + ((size_t)pol * 64 + j) * Q;
-        float2 Y = Z[(cc * Q) * WEX + m];
-        for (int bb = 1; bb < Q; bb++) Y = cadd(Y, cmul(Z[(cc * Q + bb) * WEX + m], __ldg(&tc[bb])));
+        float2 Y = Z[cc * WZ + m];
+        for (int bb = 1; bb < Q; bb++) Y = cadd(Y, cmul(Z[(bb * WC + cc) * WZ + m], __ldg(&tc[bb])));
         Y = cmul(Y, bc);
         f.window[((size_t)unit * 64 + j) * w + c0 + cc] =
             cmul(Y, __ldg(&f.tabAdj[((size_t)pol * 64 + j) * w + c0 + cc]));
@@ -306,7 +319,7 @@ cudaError_t dh_launch_plane_rows512(const DhFourierParams& q, int compact, cudaS
     }
     const int units = f.frameCount * f.polCount;
     if (units <= 0) return cudaSuccess;
-    const size_t smem = sizeof(float2) * (size_t)RR * RN;
+    const size_t smem = sizeof(float2) * ((size_t)RR * RN + RN + RN + 1);
     const unsigned blocks = (unsigned)((units * ((1 << f.logH) / RR) + NG - 1) / NG);
     if (f.inputU16) {
         k_plane_rows512<true><<<blocks, 256, smem, s>>>(q, compact);
@@ -325,7 +338,8 @@ cudaError_t dh_launch_plane_window64(const DhFourierParams& q, cudaStream_t s) {
     const int units = f.frameCount * f.polCount;
     if (units <= 0) return cudaSuccess;
     const int H = 1 << f.logH;
-    const size_t smem = sizeof(float2) * ((size_t)WC * (H + 8) + (size_t)64 * WEX);
+    const int Q = H >> 6;
+    const size_t smem = sizeof(float2) * ((size_t)WC * (H + 2 > Q * WZ ? H + 2 : Q * WZ) + (size_t)64 * WEX);
     cudaError_t e = setSmemOnce(reinterpret_cast<const void*>(k_plane_window64), (int)smem);
     if (e != cudaSuccess) return e;
     k_plane_window64<<<(unsigned)(units * (f.w / WC)), WT, smem, s>>>(q);
