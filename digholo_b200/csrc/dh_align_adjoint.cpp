@@ -26,6 +26,12 @@ static const double PI_DA = 3.14159265358979323846;
 static const float UNIT_ANGLE_A = (float)(PI_DA / 180.0);
 enum { G_TX = 0, G_TY = 1, G_DEF = 2, G_CX = 3, G_CY = 4, G_WAIST = 5 };
 
+// The gradient takes the Fourier windows of the batch where the inverse stage
+// is separable: no reference-wave calibration, whose planes multiply the
+// pixels, and one wavelength (of a sweep the device holds the last one's
+// windows only).  Otherwise it takes the float fields.
+static bool gradientFromWindow(const Object& o) { return !objRefCalApplies(o) && o.wavelengths.size() <= 1; }
+
 // grad12[pol * 6 + k], k in {tiltX, tiltY, defocus, beamCentreX, beamCentreY,
 // waist} (config units: degrees, dioptre, m, m); parameters tied by the
 // polarisation locks carry the sum on polarisation 0 and zero on 1.
@@ -50,9 +56,10 @@ int objAlignEvaluate(Object& o, int metric, int stage, float* grad12, float* ilO
     using Clock = std::chrono::steady_clock;
     const auto t0 = Clock::now();
     int r = ERR_SUCCESS;
+    const bool fromWindow = gradientFromWindow(o);
     if (stage != ALIGN_EVAL_GRADIENT) {
         const int keep = o.keepField32;
-        o.keepField32 = 1;
+        if (!fromWindow) o.keepField32 = 1;
         r = objProcessForAlign(o);
         o.keepField32 = keep;
         if (r) return r;
@@ -90,23 +97,25 @@ int objAlignEvaluate(Object& o, int metric, int stage, float* grad12, float* ilO
         }
         DH_CUDA(o, o.dGradTab.ensure(tab.size() * sizeof(float)));
         DH_CUDA(o, cudaMemcpyAsync(o.dGradTab.ptr, tab.data(), tab.size() * sizeof(float), cudaMemcpyHostToDevice, o.stream));
-        const size_t winElems = (size_t)units * w * h;
-        DH_CUDA(o, o.dGradW.ensure(2 * winElems * sizeof(float2)));
-        float2* Wx = o.dGradW.as<float2>();
-        float2* Wy = Wx + winElems;
-        DH_CUDA(o, dh_launch_window_deriv(o.dWindow.as<float2>(), o.dGradTab.as<float>(), o.dGradTab.as<float>() + (size_t)P * w,
-                                          w, h, P, units, Wx, Wy, o.stream));
-        // fields of the derivative windows
-        DH_CUDA(o, o.dGradV.ensure(2 * (size_t)units * npix * sizeof(float2)));
-        Vx = o.dGradV.as<float2>();
-        Vy = Vx + (size_t)units * npix;
-        // both derivative windows in one launch: a batch of 2B frames (Wy follows Wx, Vy follows Vx)
-        DH_CUDA(o, o.dGradScratch.ensure(4 * (size_t)units * npix * sizeof(short) + (size_t)7 * P * (2 * B + 1) * sizeof(float)));
-        short* sR = o.dGradScratch.as<short>();
-        short* sI = sR + 2 * (size_t)units * npix;
-        float* sStats = reinterpret_cast<float*>(sI + 2 * (size_t)units * npix);
-        r = objInverseAux(o, Wx, 2 * B, Vx, sR, sI, sStats);
-        if (r) return r;
+        if (!fromWindow) {
+            const size_t winElems = (size_t)units * w * h;
+            DH_CUDA(o, o.dGradW.ensure(2 * winElems * sizeof(float2)));
+            float2* Wx = o.dGradW.as<float2>();
+            float2* Wy = Wx + winElems;
+            DH_CUDA(o, dh_launch_window_deriv(o.dWindow.as<float2>(), o.dGradTab.as<float>(), o.dGradTab.as<float>() + (size_t)P * w,
+                                              w, h, P, units, Wx, Wy, o.stream));
+            // fields of the derivative windows
+            DH_CUDA(o, o.dGradV.ensure(2 * (size_t)units * npix * sizeof(float2)));
+            Vx = o.dGradV.as<float2>();
+            Vy = Vx + (size_t)units * npix;
+            // both derivative windows in one launch: a batch of 2B frames (Wy follows Wx, Vy follows Vx)
+            DH_CUDA(o, o.dGradScratch.ensure(4 * (size_t)units * npix * sizeof(short) + (size_t)7 * P * (2 * B + 1) * sizeof(float)));
+            short* sR = o.dGradScratch.as<short>();
+            short* sI = sR + 2 * (size_t)units * npix;
+            float* sStats = reinterpret_cast<float*>(sI + 2 * (size_t)units * npix);
+            r = objInverseAux(o, Wx, 2 * B, Vx, sR, sI, sStats);
+            if (r) return r;
+        }
         t2 = Clock::now();
         // float modes up to order G + 1 (the waist derivative reaches m + 2)
         const int GE = G + 2;
@@ -162,7 +171,46 @@ int objAlignEvaluate(Object& o, int metric, int stage, float* grad12, float* ilO
     }
     DH_CUDA(o, o.dGradOut.ensure((size_t)units * 7 * sizeof(float)));
     gp.out = o.dGradOut.as<float>();
-    DH_CUDA(o, valueOnly ? dh_launch_align_power(gp, o.stream) : dh_launch_align_grad(gp, o.stream));
+    if (valueOnly) {
+        DH_CUDA(o, dh_launch_align_power(gp, o.stream));
+    } else if (!fromWindow) {
+        DH_CUDA(o, dh_launch_align_grad(gp, o.stream));
+    } else {
+        DhGradWindowParams wp;
+        memset(&wp, 0, sizeof(wp));
+        DH_CUDA(o, o.dGradW.ensure(dh_grad_tables_elems(P, G, w, h) * sizeof(float2)));
+        wp.window = o.dWindow.as<float2>();
+        wp.coefs = gp.coefs;
+        wp.weights = gp.weights;
+        wp.hx = hx;
+        wp.hy = hy;
+        wp.refWaveF = o.dRefF.as<float>();
+        wp.xAxis = gp.xAxis;
+        wp.yAxis = gp.yAxis;
+        wp.kx = o.dGradTab.as<float>();
+        wp.ky = o.dGradTab.as<float>() + (size_t)P * w;
+        wp.twiddle = o.dTwiddle.as<float2>();
+        wp.tabX = o.dGradW.as<float2>();
+        wp.tabY = wp.tabX + (size_t)P * 5 * G * w;
+        auto log2of = [](int n) { int l = 0; while ((1 << l) < n) l++; return l; };
+        wp.w = w; wp.h = h; wp.logw = log2of(w); wp.logh = log2of(h);
+        wp.nx = g.nx; wp.ny = g.ny; wp.lognx = log2of(g.nx); wp.logny = log2of(g.ny);
+        wp.lowres = c.resolutionIdx;
+        wp.frameCount = B; wp.polCount = P; wp.G = G; wp.M = M;
+        for (int p = 0; p < P; p++) {
+            wp.sx0[p] = g.SX[p] - W / 2;
+            wp.sy[p] = g.SY[p];
+            wp.k0u[p] = gp.k0u[p];
+            wp.tiltX[p] = gp.tiltX[p];
+            wp.tiltY[p] = gp.tiltY[p];
+            wp.bcx[p] = gp.bcx[p];
+            wp.bcy[p] = gp.bcy[p];
+            wp.waist[p] = gp.waist[p];
+        }
+        wp.piOverLambda = gp.piOverLambda;
+        wp.out = gp.out;
+        DH_CUDA(o, dh_launch_align_grad_window(wp, o.stream));
+    }
     if (!o.hGradOut.ensure((size_t)units * 7 * sizeof(float))) return fail(o, ERR_MEMORYALLOCATION, "gradient host buffer");
     const float* part = o.hGradOut.as<float>();
     DH_CUDA(o, cudaMemcpyAsync(o.hGradOut.ptr, gp.out, (size_t)units * 7 * sizeof(float), cudaMemcpyDeviceToHost, o.stream));
@@ -267,7 +315,7 @@ float objAutoAlignAdjoint(Object& o) {
         Object& o; const void* f; int d; int k;
         ~Restore() { o.frames = f; o.framesOnDevice = d; o.keepField32 = k; o.useSnaps = 0; o.preparedValid = 0; }
     } restore{o, userFrames, userOnDevice, o.keepField32};
-    o.keepField32 = 1;   // every evaluation needs the float field for the adjoint
+    if (!gradientFromWindow(o)) o.keepField32 = 1;   // every evaluation needs the float field for the adjoint
     {
         int r0 = objProcessForAlign(o);
         if (r0) return -FLT_MAX;

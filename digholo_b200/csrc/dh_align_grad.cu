@@ -19,8 +19,10 @@
 //             i kx (the beam-centre phase of digHoloCopyWindow, digHolo.cpp:1955-2035),
 // and for the waist the Hermite-Gaussian ladder relation
 //   dpsi_m/dw = -(1 / 2w) (sqrt(m (m-1)) psi_{m-2} - sqrt((m+1)(m+2)) psi_{m+2}).
-// One block per (frame, polarisation) field; per-field partial sums of
-// Re sum conj(c) dc for the six parameters and the field's sum |c|^2.
+// Per-field partial sums of Re sum conj(c) dc for the six parameters and the
+// field's sum |c|^2, from the Fourier windows where the inverse stage is
+// separable (k_align_grad_window), else from the pixels of V, Vx and Vy, one
+// block per (frame, polarisation) field.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -432,6 +434,223 @@ __global__ void __launch_bounds__(256) k_align_grad_tile(DhGradParams p) {
     }
 }
 
+// ---------------------------------------------------------------- in the Fourier window
+// The same sums from the Fourier window W alone.  A is the inverse transform
+// of W, and the modes, the reference wave and the weights x, x^2, kx of the
+// tangents are all separable, so every sum over pixels is a sum over the
+// window:
+//   sum_xy conj(Abar) f(x) g(y) A R = sum_jc W[j][c] sum_mn c_mn F_m[c] K_n[j],
+//   F_m[c] = sum_x f(x) Hx_m(x) Rx(x) exp(2 pi i col_c x / nx),   K_n[j] alike,
+// with Abar V = -conj(conj(Abar) A R).  One small kernel makes the tables F
+// and K (five each: 1, x + bcx, x^2, kx, the waist derivative of the modes)
+// for the configuration; a field then costs about (2 w h G + 5 (w + h) G^2 / 2)
+// complex products on w h values, where the pixels cost 4 nx ny G on three
+// fields of nx ny that had to be made and stored first.
+
+// F (axis 0) or K (axis 1) of one mode and polarisation per block, summed in
+// FP64: out[axis][pol][5][G][side].
+__global__ void __launch_bounds__(256) k_grad_tables(DhGradWindowParams p) {
+    extern __shared__ double part[];                       // [256][8]
+    const int m = blockIdx.x, axis = blockIdx.y, pol = blockIdx.z, tid = threadIdx.x;
+    const int side = axis ? p.h : p.w, logn = axis ? p.logny : p.lognx, n = 1 << logn;
+    const int GE = p.G + 2;
+    const float* H = (axis ? p.hy : p.hx) + (size_t)pol * GE * n;
+    const float* R = p.refWaveF + (size_t)pol * 2 * (p.nx + p.ny) + (axis ? 2 * p.nx : 0);
+    const float* ax = axis ? p.yAxis : p.xAxis;
+    const double bc = axis ? p.bcy[pol] : p.bcx[pol];
+    const double ladder = -1.0 / (2.0 * (double)p.waist[pol]);
+    const double la = m > 1 ? ladder * sqrt((double)(m * (m - 1))) : 0.0, lb = -ladder * sqrt((double)((m + 1) * (m + 2)));
+    const float* kt = (axis ? p.ky : p.kx) + pol * side;
+    float2* out = (axis ? p.tabY : p.tabX) + (size_t)pol * 5 * p.G * side;
+    const int nf = side < 256 ? side : 256, S = 256 / nf;   // side is a power of two
+    const int q = tid / nf;
+    for (int f = tid % nf; f < side; f += nf) {
+        int col = f;
+        if (!p.lowres) col = axis ? f + p.sy[pol] + n / 2 : p.sx0[pol] + f;
+        double a[8];
+        for (int v = 0; v < 8; v++) a[v] = 0.0;
+#pragma unroll 8
+        for (int x = q; x < n; x += S) {
+            const float2 e = __ldg(&p.twiddle[((unsigned)(col * x) & (unsigned)(n - 1)) << (TW_LOG - logn)]);   // conjugate of the kernel
+            const double rr = R[x], ri = R[n + x];
+            const double tr = rr * e.x + ri * e.y, ti = ri * e.x - rr * e.y;   // Rx exp(+)
+            const double hm = H[(size_t)m * n + x];
+            const double hw = (m > 1 ? la * H[(size_t)(m - 2) * n + x] : 0.0) + lb * H[(size_t)(m + 2) * n + x];
+            const double xv = ax[x], gr = hm * tr, gi = hm * ti;
+            a[0] += gr;
+            a[1] += gi;
+            a[2] += (xv + bc) * gr;
+            a[3] += (xv + bc) * gi;
+            a[4] += xv * xv * gr;
+            a[5] += xv * xv * gi;
+            a[6] += hw * tr;
+            a[7] += hw * ti;
+        }
+        for (int v = 0; v < 8; v++) part[(size_t)v * 256 + tid] = a[v];
+        __syncthreads();
+        if (q == 0) {
+            for (int u = 1; u < S; u++)
+                for (int v = 0; v < 8; v++) a[v] += part[(size_t)v * 256 + u * nf + tid];
+            const double k = kt[f];
+            const size_t o = (size_t)m * side + f, st = (size_t)p.G * side;
+            out[o] = make_float2((float)a[0], (float)a[1]);
+            out[st + o] = make_float2((float)a[2], (float)a[3]);
+            out[2 * st + o] = make_float2((float)a[4], (float)a[5]);
+            out[3 * st + o] = make_float2((float)(k * a[0]), (float)(k * a[1]));
+            out[4 * st + o] = make_float2((float)a[6], (float)a[7]);
+        }
+        __syncthreads();
+    }
+}
+
+constexpr int GB = 3;   // blocks per SM of the window kernel (2 and 4: the same time)
+
+// Half of a field's sums, by 128 threads.  An item is one window column (row)
+// u and four modes n of the other axis, 2 i, 2 i + 1 and their mirrors
+// G - 1 - n, whose lengths G - n add up to the same for every i:
+//   Y_n = sum_v B_n[v] W(u, v)   (B the other axis's base table)
+//   s[k] += (sum_m c_mn T^k_m[u]) Y_n,   k = 1, lin, quad, k, waist.
+// XS: u = column, n the modes of y; else u = row, n those of x.  c[m][n], zero
+// for m + n >= G.
+template <bool XS>
+__device__ __forceinline__ void gradHalf(const float2* __restrict__ W, int ld, const float2* __restrict__ c, int G,
+                                         const float2* __restrict__ T, const float2* __restrict__ B, int logu, int nv,
+                                         int t, float (&s)[5]) {
+    const int nu = 1 << logu, half = (G + 1) >> 1, quads = (half + 1) >> 1;
+    const int st = G << logu;
+    for (int item = t; item < quads << logu; item += 128) {
+        const int i = item >> logu, u = item & (nu - 1);
+        const int n0 = 2 * i, n1 = min(2 * i + 1, half - 1);
+        const int n[4] = {n0, n1, G - 1 - n0, G - 1 - n1};
+        const bool use[4] = {true, n1 != n0, n[2] != n0, n1 != n0 && n[3] != n1};
+        float2 y[4];
+        const float4* b[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            y[k] = make_float2(0.f, 0.f);
+            b[k] = reinterpret_cast<const float4*>(B + (size_t)n[k] * nv);
+        }
+#pragma unroll 4
+        for (int v = 0; v < nv; v += 2) {
+            const float2 w0 = XS ? W[(size_t)v * ld + u] : W[(size_t)u * ld + v];
+            const float2 w1 = XS ? W[(size_t)(v + 1) * ld + u] : W[(size_t)u * ld + v + 1];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const float4 q = b[k][v >> 1];
+                y[k].x = fmaf(q.x, w0.x, fmaf(-q.y, w0.y, y[k].x));
+                y[k].y = fmaf(q.x, w0.y, fmaf(q.y, w0.x, y[k].y));
+                y[k].x = fmaf(q.z, w1.x, fmaf(-q.w, w1.y, y[k].x));
+                y[k].y = fmaf(q.z, w1.y, fmaf(q.w, w1.x, y[k].y));
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (!use[k]) y[k] = make_float2(0.f, 0.f);   // a mode counts once
+        // z_m = sum of c_mn Y_n over the four n serves the five tables
+        const float2* tu = T + u;
+#pragma unroll 2
+        for (int m = 0; m < G - n0; m++) {
+            const float2* cm = c + m * G;
+            float zr = 0.f, zi = 0.f;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                if (k >= 2 && m > n1) break;   // the mirrors end at m = n
+                const float2 a = cm[n[k]];
+                zr = fmaf(a.x, y[k].x, fmaf(-a.y, y[k].y, zr));
+                zi = fmaf(a.x, y[k].y, fmaf(a.y, y[k].x, zi));
+            }
+            const float2* tm = tu + (m << logu);
+            const float2 t1 = tm[st], t2 = tm[2 * st], t3 = tm[3 * st], t4 = tm[4 * st];
+            if (XS) {
+                const float2 t0 = tm[0];
+                s[0] = fmaf(t0.x, zi, fmaf(t0.y, zr, s[0]));
+            }
+            s[1] = fmaf(t1.x, zi, fmaf(t1.y, zr, s[1]));
+            s[2] = fmaf(t2.x, zi, fmaf(t2.y, zr, s[2]));
+            s[3] = fmaf(t3.x, zi, fmaf(t3.y, zr, s[3]));
+            s[4] = fmaf(t4.x, zr, fmaf(-t4.y, zi, s[4]));
+        }
+    }
+}
+
+// One (frame, polarisation) at a time per block of a fixed polarisation, the x
+// tables' sums by its first four warps, the y tables' by the others; SM: the
+// tables and the window in shared memory (this build's kernels keep the L1
+// small, so the tables would come from the L2 each time).
+// Bound: the shared-memory reads of the products (14.7 M instructions at 62 %
+// of the issue slots, 5 % of the DRAM).  1024 fields of 128 x 128 (32 x 32
+// windows), 15 groups: 28 us, and 10 for the tables (47 with one unit per block
+// and the tables in global memory); the pixel path took 10 + 108 us for the
+// derivative fields, 30 more in the batch for V and 141 for its contraction.
+template <bool SM>
+__global__ void __launch_bounds__(256, GB) k_align_grad_window(DhGradWindowParams p) {
+    extern __shared__ float4 sg4[];
+    __shared__ float red[8 * 7];
+    const int P = p.polCount, G = p.G, M = p.M, w = p.w, h = p.h;
+    const int pol = blockIdx.x % P;   // the grid is a multiple of P
+    const int tid = threadIdx.x;
+    const int nt = SM ? 5 * G * (w + h) : 0;
+    float2* st = reinterpret_cast<float2*>(sg4);   // the polarisation's tables, x then y
+    float2* c = st + nt;                           // [m][n] and [n][m]: conj of Abar's coefficients, zero for m + n >= G
+    float2* sw = c + 2 * G * G;                    // [h][w + 1]
+    const float2* tx = p.tabX + (size_t)pol * 5 * G * w;
+    const float2* ty = p.tabY + (size_t)pol * 5 * G * h;
+    if (SM) {
+        const int nx4 = 5 * G * w / 2;
+        for (int e = tid; e < nt / 2; e += 256)
+            sg4[e] = e < nx4 ? __ldg(reinterpret_cast<const float4*>(tx) + e) : __ldg(reinterpret_cast<const float4*>(ty) + e - nx4);
+    }
+    const float k0u = p.k0u[pol];
+    for (int unit = blockIdx.x; unit < p.frameCount * P; unit += gridDim.x) {
+        const int frame = unit / P;
+        const float2* win = p.window + (size_t)unit * h * w;
+        // in the order of the other gradient kernels
+        float spow = 0.f;
+        for (int mode = tid; mode < M; mode += 256) {
+            const float2 v = p.coefs[(size_t)frame * P * M + (size_t)pol * M + mode];
+            spow = fmaf(v.x, v.x, fmaf(v.y, v.y, spow));
+        }
+        const float2* src = (p.weights ? p.weights : p.coefs) + (size_t)frame * P * M + (size_t)pol * M;
+        const float sgn = p.weights ? -1.0f : 1.0f;   // conj(Abar's coefficients)
+        for (int e = tid; e < G * G; e += 256) {
+            const int n = e / G, m = e - n * G, g = m + n;
+            float2 v = make_float2(0.f, 0.f);
+            if (g < G) {
+                v = src[g * (g + 1) / 2 + n];
+                v.y *= sgn;
+            }
+            c[m * G + n] = v;
+            c[G * G + e] = v;
+        }
+        if (SM)
+            for (int e = tid; e < h * w; e += 256) sw[(e >> p.logw) * (w + 1) + (e & (w - 1))] = win[e];
+        __syncthreads();
+        float sx[5] = {0.f, 0.f, 0.f, 0.f, 0.f}, sy[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+        if (SM) {
+            if (tid < 128) gradHalf<true>(sw, w + 1, c, G, st, st + 5 * G * w, p.logw, h, tid, sx);
+            else gradHalf<false>(sw, w + 1, c + G * G, G, st + 5 * G * w, st, p.logh, w, tid - 128, sy);
+        } else {
+            if (tid < 128) gradHalf<true>(win, w, c, G, tx, ty, p.logw, h, tid, sx);
+            else gradHalf<false>(win, w, c + G * G, G, ty, tx, p.logh, w, tid - 128, sy);
+        }
+        // Im(Abar V) = Im, Re(Abar V) = -Re of the sums (Abar V = -conj of them)
+        float s[7] = {-k0u * sx[1], -k0u * sy[1], -p.piOverLambda * (sx[2] + sy[2]), sx[3] - k0u * p.tiltX[pol] * sx[0],
+                      sy[3] - k0u * p.tiltY[pol] * sx[0], -(sx[4] + sy[4]), spow};
+#pragma unroll
+        for (int k = 0; k < 7; k++)
+            for (int off = 16; off > 0; off >>= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], off);
+        if ((tid & 31) == 0)
+            for (int k = 0; k < 7; k++) red[(tid >> 5) * 7 + k] = s[k];
+        __syncthreads();   // also: c and the window are free for the next unit
+        if (tid < 7) {
+            float t = 0.f;
+            for (int wv = 0; wv < 8; wv++) t += red[wv * 7 + tid];
+            p.out[(size_t)unit * 7 + tid] = t;
+        }
+        // red is rewritten only after the next unit's first barrier
+    }
+}
+
 // The power term of the gradient kernels alone (their first loop and their
 // block reduction, in the same order).
 __global__ void __launch_bounds__(256) k_align_power(DhGradParams p) {
@@ -566,5 +785,39 @@ cudaError_t dh_launch_align_grad(const DhGradParams& p, cudaStream_t s) {
     cudaError_t e = setSmemOnce(reinterpret_cast<const void*>(k_align_grad), (int)smem);
     if (e != cudaSuccess) return e;
     k_align_grad<<<(unsigned)(p.frameCount * p.polCount), 256, smem, s>>>(p);
+    return cudaGetLastError();
+}
+
+size_t dh_grad_tables_elems(int P, int G, int w, int h) { return (size_t)P * 5 * G * (w + h); }
+
+// The refusal of the pixel kernels (fields whose row sums exceed shared
+// memory) holds here too: what can be aligned does not depend on a calibration.
+cudaError_t dh_launch_align_grad_window(const DhGradWindowParams& p, cudaStream_t s) {
+    const size_t reg = sizeof(float4) * (size_t)(p.G <= 16 ? 16 : 32) * p.ny + sizeof(float2) * (size_t)p.M +
+                       sizeof(float) * ((size_t)p.G * p.ny + 8 * 7);
+    const size_t any = sizeof(float2) * ((size_t)p.M + 2 * (size_t)p.G * p.ny) +
+                       sizeof(float) * ((size_t)p.G * (p.nx + p.ny) + 8 * 7);
+    if ((p.G > 32 || reg > 200 * 1024) && any > 200 * 1024) return cudaErrorNotSupported;
+    if (p.lognx > TW_LOG || p.logny > TW_LOG) return cudaErrorNotSupported;
+    k_grad_tables<<<dim3(p.G, 2, p.polCount), 256, 256 * 8 * sizeof(double), s>>>(p);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    const unsigned units = (unsigned)(p.frameCount * p.polCount);
+    // the base tables are read in pairs
+    if ((reinterpret_cast<uintptr_t>(p.tabX) | reinterpret_cast<uintptr_t>(p.tabY)) & 15) return cudaErrorInvalidValue;
+    const size_t cs = sizeof(float2) * 2 * (size_t)p.G * p.G;
+    const size_t ws = cs + sizeof(float2) * ((size_t)p.h * (p.w + 1) + 5 * (size_t)p.G * (p.w + p.h));
+    const bool sm = ws <= 200 * 1024;
+    unsigned grid = (unsigned)smCountCached() * GB / p.polCount * p.polCount;
+    if (grid > units) grid = units;
+    if (sm) {
+        e = setSmemOnce(reinterpret_cast<const void*>(k_align_grad_window<true>), (int)ws);
+        if (e != cudaSuccess) return e;
+        k_align_grad_window<true><<<grid, 256, ws, s>>>(p);
+    } else {
+        e = setSmemOnce(reinterpret_cast<const void*>(k_align_grad_window<false>), (int)cs);
+        if (e != cudaSuccess) return e;
+        k_align_grad_window<false><<<grid, 256, cs, s>>>(p);
+    }
     return cudaGetLastError();
 }

@@ -24,6 +24,32 @@ struct DhGradParams {
     const float2* weights;
 };
 
+// The gradient from the Fourier windows (batches without a reference-wave
+// calibration): the scalars of DhGradParams and the separable pieces of the
+// inverse stage.
+struct DhGradWindowParams {
+    const float2* window;   // [unit][h][w]
+    const float2* coefs;    // [frame][pol * M + mode]
+    const float2* weights;  // as in DhGradParams
+    const float* hx;        // [pol][G + 2][nx] float modes (unquantised)
+    const float* hy;        // [pol][G + 2][ny]
+    const float* refWaveF;  // [pol][2 (nx + ny)]: Xr, Xi, Yr, Yi
+    const float* xAxis;
+    const float* yAxis;
+    const float* kx;        // [pol][w]
+    const float* ky;        // [pol][h]
+    const float2* twiddle;
+    float2* tabX;           // scratch [pol][5][G][w]
+    float2* tabY;           // scratch [pol][5][G][h]
+    int w, h, logw, logh, nx, ny, lognx, logny, lowres;
+    int sx0[2], sy[2];      // full-resolution placement of the window
+    int frameCount, polCount, G, M;
+    float k0u[2], tiltX[2], tiltY[2], bcx[2], bcy[2], piOverLambda, waist[2];
+    float* out;             // [unit][7], as in DhGradParams
+};
+size_t dh_grad_tables_elems(int polCount, int G, int w, int h);
+cudaError_t dh_launch_align_grad_window(const DhGradWindowParams& p, cudaStream_t s);
+
 // Per field only the captured power sum |c|^2 into out[unit * 7 + 6] (the
 // other six entries zero), summed in the order of the gradient kernels, so
 // the value equals theirs bit for bit: the value of a line-search trial.
