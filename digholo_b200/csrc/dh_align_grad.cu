@@ -448,9 +448,10 @@ __global__ void __launch_bounds__(256) k_align_grad_tile(DhGradParams p) {
 // fields of nx ny that had to be made and stored first.
 
 // F (axis 0) or K (axis 1) of one mode and polarisation per block, summed in
-// FP64: out[axis][pol][5][G][side].
+// FP64: out[axis][pol][5][G][side].  The samples' factors (mode and waist
+// derivative times wave, position) are formed once, in shared memory.
 __global__ void __launch_bounds__(256) k_grad_tables(DhGradWindowParams p) {
-    extern __shared__ double part[];                       // [256][8]
+    extern __shared__ double sd[];
     const int m = blockIdx.x, axis = blockIdx.y, pol = blockIdx.z, tid = threadIdx.x;
     const int side = axis ? p.h : p.w, logn = axis ? p.logny : p.lognx, n = 1 << logn;
     const int GE = p.G + 2;
@@ -458,10 +459,24 @@ __global__ void __launch_bounds__(256) k_grad_tables(DhGradWindowParams p) {
     const float* R = p.refWaveF + (size_t)pol * 2 * (p.nx + p.ny) + (axis ? 2 * p.nx : 0);
     const float* ax = axis ? p.yAxis : p.xAxis;
     const double bc = axis ? p.bcy[pol] : p.bcx[pol];
-    const double ladder = -1.0 / (2.0 * (double)p.waist[pol]);
-    const double la = m > 1 ? ladder * sqrt((double)(m * (m - 1))) : 0.0, lb = -ladder * sqrt((double)((m + 1) * (m + 2)));
     const float* kt = (axis ? p.ky : p.kx) + pol * side;
     float2* out = (axis ? p.tabY : p.tabX) + (size_t)pol * 5 * p.G * side;
+    double* part = sd;                                     // [8][256]
+    double2* tw = reinterpret_cast<double2*>(sd + 8 * 256);   // [n] exp(+2 pi i x / n)
+    float4* smp = reinterpret_cast<float4*>(tw + n);       // [n] {mode, derivative, Rr, Ri}
+    float* pos = reinterpret_cast<float*>(smp + n);        // [n]
+    {
+        const double ladder = -1.0 / (2.0 * (double)p.waist[pol]);
+        const double la = m > 1 ? ladder * sqrt((double)(m * (m - 1))) : 0.0, lb = -ladder * sqrt((double)((m + 1) * (m + 2)));
+        for (int x = tid; x < n; x += 256) {
+            const float2 e = __ldg(&p.twiddle[x << (TW_LOG - logn)]);
+            tw[x] = make_double2(e.x, -e.y);
+            const double hw = (m > 1 ? la * H[(size_t)(m - 2) * n + x] : 0.0) + lb * H[(size_t)(m + 2) * n + x];
+            smp[x] = make_float4(H[(size_t)m * n + x], (float)hw, R[x], R[n + x]);
+            pos[x] = ax[x];
+        }
+    }
+    __syncthreads();
     const int nf = side < 256 ? side : 256, S = 256 / nf;   // side is a power of two
     const int q = tid / nf;
     for (int f = tid % nf; f < side; f += nf) {
@@ -469,22 +484,21 @@ __global__ void __launch_bounds__(256) k_grad_tables(DhGradWindowParams p) {
         if (!p.lowres) col = axis ? f + p.sy[pol] + n / 2 : p.sx0[pol] + f;
         double a[8];
         for (int v = 0; v < 8; v++) a[v] = 0.0;
-#pragma unroll 8
+#pragma unroll 4
         for (int x = q; x < n; x += S) {
-            const float2 e = __ldg(&p.twiddle[((unsigned)(col * x) & (unsigned)(n - 1)) << (TW_LOG - logn)]);   // conjugate of the kernel
-            const double rr = R[x], ri = R[n + x];
-            const double tr = rr * e.x + ri * e.y, ti = ri * e.x - rr * e.y;   // Rx exp(+)
-            const double hm = H[(size_t)m * n + x];
-            const double hw = (m > 1 ? la * H[(size_t)(m - 2) * n + x] : 0.0) + lb * H[(size_t)(m + 2) * n + x];
-            const double xv = ax[x], gr = hm * tr, gi = hm * ti;
+            const double2 e = tw[(unsigned)(col * x) & (unsigned)(n - 1)];
+            const float4 s = smp[x];
+            const double rr = s.z, ri = s.w;
+            const double tr = rr * e.x - ri * e.y, ti = ri * e.x + rr * e.y;   // Rx exp(+)
+            const double xv = pos[x], gr = s.x * tr, gi = s.x * ti;
             a[0] += gr;
             a[1] += gi;
             a[2] += (xv + bc) * gr;
             a[3] += (xv + bc) * gi;
             a[4] += xv * xv * gr;
             a[5] += xv * xv * gi;
-            a[6] += hw * tr;
-            a[7] += hw * ti;
+            a[6] += s.y * tr;
+            a[7] += s.y * ti;
         }
         for (int v = 0; v < 8; v++) part[(size_t)v * 256 + tid] = a[v];
         __syncthreads();
@@ -579,8 +593,9 @@ __device__ __forceinline__ void gradHalf(const float2* __restrict__ W, int ld, c
 // small, so the tables would come from the L2 each time).
 // Bound: the shared-memory reads of the products (14.7 M instructions at 62 %
 // of the issue slots, 5 % of the DRAM).  1024 fields of 128 x 128 (32 x 32
-// windows), 15 groups: 28 us, and 10 for the tables (47 with one unit per block
-// and the tables in global memory); the pixel path took 10 + 108 us for the
+// windows), 15 groups: 28 us, and 7 for the tables (47 with one unit per block
+// and the tables in global memory, 11 with each table's samples fetched in its
+// loop); the pixel path took 10 + 108 us for the
 // derivative fields, 30 more in the batch for V and 141 for its contraction.
 template <bool SM>
 __global__ void __launch_bounds__(256, GB) k_align_grad_window(DhGradWindowParams p) {
@@ -799,8 +814,11 @@ cudaError_t dh_launch_align_grad_window(const DhGradWindowParams& p, cudaStream_
                        sizeof(float) * ((size_t)p.G * (p.nx + p.ny) + 8 * 7);
     if ((p.G > 32 || reg > 200 * 1024) && any > 200 * 1024) return cudaErrorNotSupported;
     if (p.lognx > TW_LOG || p.logny > TW_LOG) return cudaErrorNotSupported;
-    k_grad_tables<<<dim3(p.G, 2, p.polCount), 256, 256 * 8 * sizeof(double), s>>>(p);
-    cudaError_t e = cudaGetLastError();
+    const size_t ts = 256 * 8 * sizeof(double) + (sizeof(double2) + sizeof(float4) + sizeof(float)) * (size_t)(p.nx > p.ny ? p.nx : p.ny);
+    cudaError_t e = setSmemOnce(reinterpret_cast<const void*>(k_grad_tables), (int)ts);
+    if (e != cudaSuccess) return e;
+    k_grad_tables<<<dim3(p.G, 2, p.polCount), 256, ts, s>>>(p);
+    e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     const unsigned units = (unsigned)(p.frameCount * p.polCount);
     // the base tables are read in pairs

@@ -566,8 +566,9 @@ struct DhBasisJobs {
 // maximum, then for the scaled values, so that a chunk costs two barriers
 // instead of three per mode; its coefficients are formed once, one mode per
 // thread.  Bound: the latency of the FP64 recurrence (one sample per thread
-// up to 1024).  Four axes of 128 samples, 17 modes: 19 us; 44 us when a thread
-// took four samples and every mode its own barriers and coefficients.
+// up to 1024).  Four axes of 128 samples, 17 modes: 19 us, 12 when only
+// the float modes are wanted (the gradient), which need no maximum; 44 us when
+// a thread took four samples and every mode its own barriers and coefficients.
 __global__ void __launch_bounds__(1024) k_basis(DhBasisJobs jobs) {
     const DhBasisParams& p = jobs.job[blockIdx.x];
     constexpr int CHUNK = 64;
@@ -623,7 +624,7 @@ __global__ void __launch_bounds__(1024) k_basis(DhBasisJobs jobs) {
         double t0[PER], t1[PER];
 #pragma unroll
         for (int q = 0; q < PER; q++) { t0[q] = h0[q]; t1[q] = h1[q]; }
-        for (int i = 0; i < count; i++) {
+        for (int i = 0; m0 < p.modes16 && i < count; i++) {   // float modes alone need no maximum
             double m = 0.0;
 #pragma unroll
             for (int q = 0; q < PER; q++)
@@ -633,7 +634,7 @@ __global__ void __launch_bounds__(1024) k_basis(DhBasisJobs jobs) {
             if ((threadIdx.x & 31) == 0) atomicMax(&maxBits[i], (unsigned long long)__double_as_longlong(m));
         }
         __syncthreads();
-        for (int i = threadIdx.x; i < count; i += blockDim.x) {
+        for (int i = threadIdx.x; m0 < p.modes16 && i < count; i += blockDim.x) {
             const double sf = 32767.0 / __longlong_as_double((long long)maxBits[i]);
             scale[i] = (float)sf;
             if (m0 + i < p.modes16) p.scale[m0 + i] = (float)(1.0 / sf);
