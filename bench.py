@@ -53,7 +53,7 @@ def parse():
     ap.add_argument("--mode", type=int, default=RES_MODE, help="IFFT resolution mode (0 full, 1 window)")
     ap.add_argument("--frames", type=int, default=FRAMES)
     ap.add_argument("--overlap", default="tc", choices=["tc", "f32"],
-                    help="overlap of full-resolution fields: split-BF16 tensor cores or FP32 CUDA cores")
+                    help="overlap of full-resolution fields: tensor cores or FP32 CUDA cores")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-autoalign", action="store_true", help="skip the AutoAlign (plain vs adjoint) measurement")
     ap.add_argument("--inverse-kernel", type=int, default=0,
@@ -446,7 +446,7 @@ def main():
     # kernels per step: forward + inverse, plus the separate FP32 overlap
     # kernel for full-resolution fields when that path is chosen
     per_step = 2 + (1 if (L.digHoloB200GetInverseKernel(h) == 3 and L.digHoloB200GetOverlapKernel(h) == 1) else 0)
-    overlap_name = {1: "fp32 cuda cores", 2: "split-bf16 tensor cores"}.get(L.digHoloB200GetOverlapKernel(h), "?")
+    overlap_name = {1: "fp32 cuda cores", 2: "integer tensor cores" if args.mode == 0 else "tensor cores"}.get(L.digHoloB200GetOverlapKernel(h), "?")
 
     # roofline of the dominant kernel (HBM bytes it must move per launch)
     peak, peak_kind = measured_peaks()
@@ -457,7 +457,7 @@ def main():
     inv_bytes = B * (P * w * hh * 8 + P * nx * ny * 4 + P * M * 8 + 7 * P * 4)
     fwd_name = {1: "k_forward", 2: "k_forward_reg", 3: "k_forward_tma", 4: "k_forward_i8"}.get(
         L.digHoloB200GetForwardKernel(h), "k_forward")
-    inv_name = {1: "k_inverse", 2: "k_inverse_lo16q" if w == 16 else "k_inverse_lo", 3: "k_field_full",
+    inv_name = {1: "k_inverse", 2: "k_inverse_lo16q" if w == 16 else "k_inverse_lo", 3: "k_field128" if nx == 128 and ny == 128 else "k_field_full",
                 4: "k_field_big"}.get(L.digHoloB200GetInverseKernel(h), "k_inverse")
     if fwd_ms >= inv_ms:
         kname, kbytes, kms = fwd_name, fwd_bytes, fwd_ms / max(timed, 1)
@@ -536,9 +536,10 @@ def main():
 def largefield_leg(L, torch, device, stream, no_cpu, frames=256):
     """frames/s on the large-field workload: 256 frames of 2048x2048 uint16,
     two polarisations, FFT window 512x512, full resolution (IFFT mode 0,
-    the reference's default: 512x512 fields by the band kernels), maxMG 30
+    the reference's default: 512x512 fields by k_cols512 and k_field512), maxMG 30
     (465 modes), waist 600 um, 20 dB SNR, 1/(group+1) coefficient taper; the
-    overlap in split-BF16 on the tensor cores and in FP32 on the CUDA cores.
+    overlap on the tensor cores (key split_bf16: its first precision, exact
+    integer products today) and in FP32 on the CUDA cores.
     Two device-resident batches (2.1 GB each, beyond L2) alternate; CUDA
     events on the library's stream; 3 warm-up and 5 timed batches each."""
     import ctypes as C

@@ -771,8 +771,8 @@ int digHoloB200SetInverseKernel(int h, int kernel) {
     return dh::ERR_SUCCESS;
 }
 // Inverse kernel used by the last batch: 1 block per unit, 2 warp per unit,
-// 3 full-resolution field kernel + overlap kernel, 4 full-resolution bands,
-// 5 fused into the tensor-core forward kernel.
+// 3 full-resolution field kernel, 4 full-resolution bands (or 48-pixel windows),
+// 5 fused into the tensor-core forward kernel, 6 direct DFT, 7 512-wide fields.
 int digHoloB200GetInverseKernel(int h) {
     OBJ_OR(h, 0);
     return o->lastInverseKernel;
@@ -783,13 +783,13 @@ int digHoloB200SetOverlapKernel(int h, int kernel) {
     o->overlapKernel = kernel;
     return dh::ERR_SUCCESS;
 }
-// Overlap used by the last batch: 1 FP32 CUDA cores, 2 split-BF16 tensor cores.
+// Overlap used by the last batch: 1 FP32 CUDA cores, 2 or 3 tensor cores.
 int digHoloB200GetOverlapKernel(int h) {
     OBJ_OR(h, 0);
     return o->lastOverlapKernel;
 }
 // Forward kernel used by the last batch: 1 generic, 2 register, 3 TMA-fed,
-// 4 tensor-core row DFT (uint16 frames), 5 full planes.
+// 4 tensor-core row DFT (uint16 frames), 5 planes or their one-launch form.
 int digHoloB200GetForwardKernel(int h) {
     OBJ_OR(h, 0);
     return o->lastForwardKernel;

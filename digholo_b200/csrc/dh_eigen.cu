@@ -810,7 +810,7 @@ static int ensureWork(DhEigen& e, size_t need) {
     return 0;
 }
 
-// Largest matrix the one-CTA solver takes (its shared memory).
+// Largest matrix the solvers take (k_heev's shared memory).
 int dh_eigen_max_n() { return 2048; }
 
 // `count` Hermitian n x n matrices G (column-major, consecutive, overwritten):

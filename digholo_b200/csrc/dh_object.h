@@ -208,8 +208,8 @@ struct Object {
     // low-resolution fields, else the block kernel), 1 block kernel
     int inverseKernel = 0;
     int lastInverseKernel = 0;
-    // overlap of full-resolution fields: 0 tensor cores (split-BF16) where the
-    // shape allows, 1 FP32 CUDA cores; and the one that ran last (1 FP32, 2 tensor)
+    // overlap of full-resolution fields: 0 tensor cores where the shape
+    // allows, 1 FP32 CUDA cores; and the one that ran last (1 FP32, 2 or 3 tensor)
     int overlapKernel = 0;
     int lastOverlapKernel = 0;
     int quietErrors = 0;                // kernel planner trials: launch failures are expected, not printed

@@ -458,13 +458,14 @@ int digHoloB200GetGeometry(int handleIdx, int* out10);
  * 1 generic shared-memory kernel, 2 register kernel, 3 TMA-fed kernel only,
  * 4 tensor-core row-DFT kernel only (uint16 frames, 128-row FFT windows 64
  * or 128 wide, 16- or 32-pixel IFFT windows), 5 R2C planes (rows, then
- * columns, then the window; automatic for windows 256 pixels wide or more;
- * 512-pixel rows by a register transform and, for 64-row IFFT windows, only
- * the window's columns and rows computed);
+ * columns, then the window; automatic for the windows 1 to 4 leave; FFT
+ * windows 128 or 256 pixels wide in one launch without the planes, 512-pixel
+ * rows by a register transform and, for 64-row IFFT windows, only the
+ * window's columns and rows computed);
  * the batch fails where the chosen kernel does not apply. */
 int digHoloB200SetForwardKernel(int handleIdx, int kernel);
 /* Forward kernel the last batch ran: 1 generic, 2 register, 3 TMA-fed,
- * 4 tensor-core row DFT, 5 full planes. */
+ * 4 tensor-core row DFT, 5 planes or their one-launch form. */
 int digHoloB200GetForwardKernel(int handleIdx);
 /* Inverse kernel choice (testing aid): 0 automatic (one warp per frame and
  * polarisation for 16- and 32-pixel low-resolution fields; for
@@ -483,14 +484,18 @@ int digHoloB200SetInverseKernel(int handleIdx, int kernel);
  * quantising pass with the overlap, coefficient sum), 5 fused into the
  * tensor-core forward kernel (inverse choice 3), 6 low-resolution fields
  * whose sides are multiples of 16 but not powers of two (direct DFT),
- * 7 full-resolution 64-point bands (512-wide fields, IFFT windows up to
- * 64 x 64). */
+ * 7 full-resolution fields 512 pixels wide with IFFT windows up to 64 x 64
+ * (column stage, statistics pass, quantising pass with the overlap).
+ * 128 x 128 fields run one kernel whatever the number: 3 with 16- and
+ * 32-pixel IFFT windows, 4 with 48-pixel ones. */
 int digHoloB200GetInverseKernel(int handleIdx);
-/* Overlap of full-resolution fields: 0 (default) on the tensor cores in
- * split-BF16 precision (bf16 hi + lo of both int16 operands, three products,
- * FP32 accumulation) where the field shape allows, 1 FP32 on the CUDA cores. */
+/* Overlap of full-resolution fields: 0 (default) on the tensor cores where the
+ * field shape allows (128 x 128 and 512-wide fields: exact integer products of
+ * the bytes of both int16 operands; others: split-BF16, bf16 hi + lo of both,
+ * three products, FP32 accumulation), 1 FP32 on the CUDA cores. */
 int digHoloB200SetOverlapKernel(int handleIdx, int kernel);
-/* Overlap the last batch ran: 1 FP32 CUDA cores, 2 split-BF16 tensor cores. */
+/* Overlap the last batch ran: 1 FP32 CUDA cores, 2 tensor cores, 3 tensor cores
+ * (512-wide fields). */
 int digHoloB200GetOverlapKernel(int handleIdx);
 
 /* Message of the handle's last error ("" when none). */
