@@ -319,6 +319,7 @@ __global__ void __launch_bounds__(NT, 1)
         }
     };
     int unit = blockIdx.x;
+    dependentWait();
     if (unit < units) fetchWindow(unit);
     cpAsyncWait();
     __syncthreads();
@@ -699,8 +700,7 @@ cudaError_t launchF(const DhInvParams& p, cudaStream_t s) {
     int grid = smCountCached();
     grid -= grid % p.polCount;   // a block keeps its polarisation
     if (grid > units) grid = units;
-    kern<<<(unsigned)grid, NT, L.total, s>>>(mapR, mapI, p, units);
-    return cudaGetLastError();
+    return launchDependent(kern, (unsigned)grid, NT, L.total, s, p.afterForward != 0, mapR, mapI, p, units);
 }
 
 template <int F>

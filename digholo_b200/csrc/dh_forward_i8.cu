@@ -415,6 +415,7 @@ __global__ void __launch_bounds__(64 + 128 * NG, 1) k_forward_i8(const __grid_co
     static_assert(4 * NPAD * NB <= TMEMCOLS, "accumulator sets exceed tensor memory");
 
     extern __shared__ unsigned char smRaw[];
+    releaseDependent();
     unsigned char* base = reinterpret_cast<unsigned char*>(
         (reinterpret_cast<uintptr_t>(smRaw) + 1023) & ~static_cast<uintptr_t>(1023));
     const int GI = FUSE ? ip.maxMG : 0;

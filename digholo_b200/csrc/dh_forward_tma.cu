@@ -213,6 +213,7 @@ __global__ void __launch_bounds__(256, 2) k_forward_tma(const __grid_constant__ 
     constexpr int w = HW, h = HW;
     constexpr int Q = H / HW;
     extern __shared__ unsigned char smRaw[];
+    releaseDependent();
     const int P = p.polCount;
     const int tid = threadIdx.x;
     constexpr unsigned tileBytes = (unsigned)H * ROWB;

@@ -53,6 +53,24 @@ inline int smCountCached() {
     return n;
 }
 
+// A launch that, where `early`, may start its blocks before the kernel ahead of
+// it in the stream has ended (the kernel waits by dependentWait).
+template <typename... Par, typename... Arg>
+inline cudaError_t launchDependent(void (*kern)(Par...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, bool early,
+                                   const Arg&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = early ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
 inline PFN_cuTensorMapEncodeTiled_v12000 tensorMapEncoder() {
     static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
     static std::once_flag once;

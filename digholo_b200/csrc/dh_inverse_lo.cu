@@ -141,6 +141,7 @@ __global__ void __launch_bounds__(32 * LO_WARPS) k_inverse_lo(DhInvParams p) {
         modeMN[mode] = ((g - n) << 16) | n;
     }
     __syncthreads();
+    dependentWait();
 
     const int lane = threadIdx.x & 31;
     const int ln = lane & (L - 1);
@@ -158,7 +159,7 @@ __global__ void __launch_bounds__(32 * LO_WARPS) k_inverse_lo(DhInvParams p) {
         const float4* src = reinterpret_cast<const float4*>(p.window + ((size_t)unit * L + ln) * L);
 #pragma unroll
         for (int q = 0; q < L / 2; q++) {
-            const float4 t = __ldg(src + q);
+            const float4 t = src[q];
             v[2 * q] = make_float2(t.x, t.y);
             v[2 * q + 1] = make_float2(t.z, t.w);
         }
@@ -370,18 +371,6 @@ __global__ void __launch_bounds__(Q_THREADS) k_inverse_lo16q(DhInvParams p) {
     const bool active = unit < units;
     const int pol = active ? unit % P : 0, frame = active ? unit / P : 0;
 
-    // 0. this thread's window values first (their loads overlap the tables):
-    //    row `line`, columns q + 4a
-    float2 x[4];
-    if (active) {
-        const float2* src = p.window + ((size_t)unit * L + line) * L + q;
-#pragma unroll
-        for (int a = 0; a < 4; a++) x[a] = __ldg(src + 4 * a);
-    } else {
-#pragma unroll
-        for (int a = 0; a < 4; a++) x[a] = make_float2(0.f, 0.f);
-    }
-
     float* hx = smf;
     float* hy = hx + P * G * HLD;
     float* yax = hy + P * G * HLD;
@@ -417,6 +406,19 @@ __global__ void __launch_bounds__(Q_THREADS) k_inverse_lo16q(DhInvParams p) {
         const int n = mode - g * (g + 1) / 2;
         modeMN[mode] = ((g - n) << 16) | n;
     }
+    // 0. this thread's window values, once the forward stage has written them:
+    //    row `line`, columns q + 4a
+    dependentWait();
+    float2 x[4];
+    if (active) {
+        const float2* src = p.window + ((size_t)unit * L + line) * L + q;
+#pragma unroll
+        for (int a = 0; a < 4; a++) x[a] = src[4 * a];
+    } else {
+#pragma unroll
+        for (int a = 0; a < 4; a++) x[a] = make_float2(0.f, 0.f);
+    }
+
     float2 tw[4];
     tw[0] = make_float2(1.f, 0.f);
     tw[1] = q == 0 ? w16(0) : (q == 1 ? w16(1) : (q == 2 ? w16(2) : w16(3)));
@@ -595,14 +597,12 @@ cudaError_t dh_launch_inverse_lo(const DhInvParams& p, cudaStream_t s) {
         if (smemQ > 200 * 1024) return cudaErrorNotSupported;
         e = setSmemOnce(reinterpret_cast<const void*>(k_inverse_lo16q), (int)smemQ);
         if (e != cudaSuccess) return e;
-        k_inverse_lo16q<<<(unsigned)((units + Q_UNITS - 1) / Q_UNITS), Q_THREADS, smemQ, s>>>(q);
-        return cudaGetLastError();
+        return launchDependent(k_inverse_lo16q, (unsigned)((units + Q_UNITS - 1) / Q_UNITS), Q_THREADS, smemQ, s, p.afterForward != 0, q);
     }
     const size_t smem = tables + sizeof(float2) * (size_t)UPB * L * (ULD > L + 1 ? ULD : L + 1);
     if (smem > 200 * 1024) return cudaErrorNotSupported;
     const unsigned blocks = (unsigned)((units + UPB - 1) / UPB);
     e = setSmemOnce(reinterpret_cast<const void*>(k_inverse_lo<32>), (int)smem);
     if (e != cudaSuccess) return e;
-    k_inverse_lo<32><<<blocks, 32 * LO_WARPS, smem, s>>>(q);
-    return cudaGetLastError();
+    return launchDependent(k_inverse_lo<32>, blocks, 32 * LO_WARPS, smem, s, p.afterForward != 0, q);
 }

@@ -1043,6 +1043,7 @@ static int launchChunk(Object& o, const DhFwdParams& fp0, const DhInvParams& ip0
     cudaError_t fe = launchForward(o, fp);
     if (fe != cudaSuccess) return failCuda(o, fe, "forward kernel launch");
     if (timed) DH_CUDA(o, cudaEventRecord(ev[1], o.stream));
+    ip.afterForward = !timed;
     if (ip0.fieldR) DH_CUDA(o, launchInverse(o, ip));
     if (timed) DH_CUDA(o, cudaEventRecord(ev[2], o.stream));
     return ERR_SUCCESS;
@@ -1082,7 +1083,9 @@ static int launchAveraged(Object& o, const DhFwdParams& fp0, const DhInvParams& 
     DH_CUDA(o, dh_launch_average_windows(fp.window, fp0.window, B, A, o.cfg.avgMode, P, (int)n, fp0.batchCal,
                                          fp0.batchCalCount, o.stream));
     if (ev) DH_CUDA(o, cudaEventRecord(ev[1], o.stream));
-    if (ip.fieldR) DH_CUDA(o, launchInverse(o, ip));
+    DhInvParams next = ip;
+    next.afterForward = !ev;
+    if (ip.fieldR) DH_CUDA(o, launchInverse(o, next));
     if (ev) DH_CUDA(o, cudaEventRecord(ev[2], o.stream));
     return ERR_SUCCESS;
 }

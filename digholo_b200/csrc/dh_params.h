@@ -85,6 +85,10 @@ struct DhInvParams {
     // 1: only field32 is wanted (the adjoint's derivative fields); kernels
     // that honour it skip the int16 planes (fieldR, fieldI are then unused)
     int fieldsOnly;
+    // 1: the launch directly ahead in the stream is the forward stage's (or the
+    // averaging) kernel that writes `window`, and all other inputs were
+    // complete before that one started: the kernel may start under its tail
+    int afterForward;
 };
 
 // Separable DFT stage of the calibration planes: out[u][a][b] =
