@@ -917,10 +917,12 @@ __global__ void __launch_bounds__(256) k_average_windows(const float2* __restric
 // each, 9.9 us with two (12.4 with eight and no barrier), the whole call 39.2
 // -> 35.5 us.
 template <int AV>
-__global__ void __launch_bounds__(512) k_average_windows_reg(const float2* __restrict__ in, float2* __restrict__ out,
+__global__ void __launch_bounds__(512) k_average_windows_reg(const float2* in, float2* __restrict__ out,
                                                              int batch, int avg, int mode, int polCount, int n,
                                                              const float2* __restrict__ cal, int calCount) {
     __shared__ double red[2][2][16];
+    releaseDependent();
+    dependentWait();
     const int b = blockIdx.x / polCount, pol = blockIdx.x - b * polCount;
     const float inv = (float)(1.0 / avg);
     const int T = blockDim.x, t = threadIdx.x, lane = t & 31, warp = t >> 5, warps = T >> 5;
@@ -975,15 +977,14 @@ __global__ void __launch_bounds__(512) k_average_windows_reg(const float2* __res
 }
 
 cudaError_t dh_launch_average_windows(const float2* in, float2* out, int batch, int avg, int mode, int polCount,
-                                      int n, const float2* cal, int calCount, cudaStream_t s) {
+                                      int n, const float2* cal, int calCount, int afterForward, cudaStream_t s) {
     if (batch <= 0 || polCount <= 0 || n <= 0) return cudaSuccess;
     if (avg < 1 || mode < 0 || mode > 2) return cudaErrorInvalidValue;
     if (n <= 512 * 8) {
         const int av = n <= 512 * 2 ? 2 : 8;   // two as far as 512 threads reach
         const int threads = (n + 32 * av - 1) / (32 * av) * 32;
-        if (av == 2) k_average_windows_reg<2><<<batch * polCount, threads, 0, s>>>(in, out, batch, avg, mode, polCount, n, cal, calCount);
-        else k_average_windows_reg<8><<<batch * polCount, threads, 0, s>>>(in, out, batch, avg, mode, polCount, n, cal, calCount);
-        return cudaGetLastError();
+        return launchDependent(av == 2 ? k_average_windows_reg<2> : k_average_windows_reg<8>, (unsigned)(batch * polCount),
+                               (unsigned)threads, 0, s, afterForward != 0, in, out, batch, avg, mode, polCount, n, cal, calCount);
     }
     k_average_windows<<<batch * polCount, 256, 0, s>>>(in, out, batch, avg, mode, polCount, n, cal, calCount);
     return cudaGetLastError();

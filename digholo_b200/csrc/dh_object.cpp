@@ -57,7 +57,7 @@ cudaError_t dh_launch_fields_to_c64(const short* R, const short* I, const float*
 cudaError_t dh_launch_batchsum(const short* R, const short* I, const float* stats, int statsStride,
                                int polCount, int frameCount, int npix, float* out, cudaStream_t s);
 cudaError_t dh_launch_average_windows(const float2* in, float2* out, int batch, int avg, int mode, int polCount,
-                                      int n, const float2* cal, int calCount, cudaStream_t s);
+                                      int n, const float2* cal, int calCount, int afterForward, cudaStream_t s);
 
 namespace dh {
 
@@ -1081,7 +1081,7 @@ static int launchAveraged(Object& o, const DhFwdParams& fp0, const DhInvParams& 
     cudaError_t fe = launchForward(o, fp);
     if (fe != cudaSuccess) return failCuda(o, fe, "forward kernel launch");
     DH_CUDA(o, dh_launch_average_windows(fp.window, fp0.window, B, A, o.cfg.avgMode, P, (int)n, fp0.batchCal,
-                                         fp0.batchCalCount, o.stream));
+                                         fp0.batchCalCount, !ev, o.stream));
     if (ev) DH_CUDA(o, cudaEventRecord(ev[1], o.stream));
     DhInvParams next = ip;
     next.afterForward = !ev;
