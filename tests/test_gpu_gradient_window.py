@@ -50,6 +50,7 @@ def _close(a, b):
     dict(groups=16, carrier=0.55), dict(groups=20, carrier=0.55, dtype="uint16"), dict(groups=5, pols=1),
     dict(groups=6, mode=1), dict(groups=9, mode=1, carrier=0.55), dict(groups=6, window=64, width=320, height=256, pols=1),
     dict(groups=8, window=256, width=1280, height=1024), dict(groups=9, average=2),
+    dict(groups=15, window=512, width=2048, height=2048, carrier=0.55, frames=2),   # tables and window beyond shared memory
 ], ids=lambda o: "-".join("%s%s" % kv for kv in o.items()))
 def test_against_fields(cases, over):
     c = _case(**over)
