@@ -85,7 +85,8 @@ int objMdlWeights(Object& o, float2* W, double* mdlDb) {
     const int n = rowsGram ? rows : B;
     const size_t aElems = (size_t)rows * B;
     if (o.dMetricA.ensure((size_t)K * aElems * sizeof(float2)) != cudaSuccess) return ERR_MEMORYALLOCATION;
-    const size_t gBytes = (size_t)K * n * n * 16, wBytes = (size_t)K * n * sizeof(double), vBytes = (size_t)K * 2 * n * 16;
+    // the eigenvectors behind the eigenvalues are double2: 16-byte aligned for odd K n too
+    const size_t gBytes = (size_t)K * n * n * 16, wBytes = ((size_t)K * n + 1) / 2 * 16, vBytes = (size_t)K * 2 * n * 16;
     if (o.dMetricG.ensure(gBytes + wBytes + vBytes) != cudaSuccess) return ERR_MEMORYALLOCATION;
     char* gb = o.dMetricG.as<char>();
     double* dW = reinterpret_cast<double*>(gb + gBytes);
