@@ -15,6 +15,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <functional>
 #include <vector>
 
 #include "dh_grad.h"
@@ -28,9 +29,8 @@ enum { G_TX = 0, G_TY = 1, G_DEF = 2, G_CX = 3, G_CY = 4, G_WAIST = 5 };
 
 // The gradient takes the Fourier windows of the batch where the inverse stage
 // is separable: no reference-wave calibration, whose planes multiply the
-// pixels, and one wavelength (of a sweep the device holds the last one's
-// windows only).  Otherwise it takes the float fields.
-static bool gradientFromWindow(const Object& o) { return !objRefCalApplies(o) && o.wavelengths.size() <= 1; }
+// pixels.  Otherwise it takes the float fields.
+static bool gradientFromWindow(const Object& o) { return !objRefCalApplies(o); }
 
 // grad12[pol * 6 + k], k in {tiltX, tiltY, defocus, beamCentreX, beamCentreY,
 // waist} (config units: degrees, dioptre, m, m); parameters tied by the
@@ -45,108 +45,38 @@ int objAlignGradientMetric(Object& o, int metric, float* grad12, float* ilOut) {
     return objAlignEvaluate(o, metric, ALIGN_EVAL_FULL, grad12, ilOut);
 }
 
-// stage ALIGN_EVAL_FULL: the batch, the metric and its gradient;
-// ALIGN_EVAL_VALUE: the batch and the metric only (grad12 untouched);
-// ALIGN_EVAL_GRADIENT: the gradient (and the metric) of the batch state a
-// preceding ALIGN_EVAL_VALUE call left on the device, for the same metric.
-// The metric is the same number in every stage.
-int objAlignEvaluate(Object& o, int metric, int stage, float* grad12, float* ilOut) {
-    Config& c = o.cfg;
-    if (c.maxMG <= 0) return fail(o, ERR_ERROR, "adjoint AutoAlign needs a modal basis (maxMG > 0)");
-    using Clock = std::chrono::steady_clock;
-    const auto t0 = Clock::now();
-    int r = ERR_SUCCESS;
-    const bool fromWindow = gradientFromWindow(o);
-    if (stage != ALIGN_EVAL_GRADIENT) {
-        const int keep = o.keepField32;
-        if (!fromWindow) o.keepField32 = 1;
-        r = objProcessForAlign(o);
-        o.keepField32 = keep;
-        if (r) return r;
-    }
-    const bool valueOnly = stage == ALIGN_EVAL_VALUE;
-    const auto t1 = Clock::now();
+using Clock = std::chrono::steady_clock;
+
+// What a gradient needs of the last batch's geometry and basis.
+static int gradientShape(Object& o) {
     const Geometry& g = o.geo;
     if ((g.w & (g.w - 1)) || (g.h & (g.h - 1)))
         return fail(o, ERR_INVALIDDIMENSION, "the adjoint AutoAlign needs power-of-two IFFT window sides on this build");
     if (o.basisActive)
         return fail(o, ERR_INVALIDARGUMENT, "the adjoint AutoAlign works on Hermite-Gaussian coefficients (basis type 0)");
-    const int P = o.polCount, B = o.batchCount, G = c.maxMG, M = o.modeCount;
-    const int units = B * P;
-    const int w = g.w, h = g.h, W = g.W, H = g.H;
-    const size_t npix = (size_t)g.nx * g.ny;
+    return ERR_SUCCESS;
+}
 
+// The scalars of the gradient kernels for the batch on the device: frames of
+// one wavelength, o.cfg.wavelengthCentre.
+static DhGradParams gradientParams(const Object& o, const float2* weights, float* out) {
+    const Config& c = o.cfg;
     DhGradParams gp;
     memset(&gp, 0, sizeof(gp));
-    float2* Vx = nullptr;
-    float2* Vy = nullptr;
-    float* hx = nullptr;
-    float* hy = nullptr;
-    auto t2 = t1, t3 = t1;
-    if (!valueOnly) {
-        // beam-centre phase derivatives of the window: i kx per column, i ky per row
-        std::vector<float> tab((size_t)P * (w + h));
-        for (int p = 0; p < P; p++) {
-            const int sx0 = g.SX[p] - W / 2;
-            for (int cc = 0; cc < w; cc++) tab[(size_t)p * w + cc] = g.kx[sx0 + cc];
-            for (int j = 0; j < h; j++) {
-                int row = (j + g.SY[p] + H / 2) % H;
-                if (row < 0) row += H;
-                tab[(size_t)P * w + (size_t)p * h + j] = g.ky[row];
-            }
-        }
-        DH_CUDA(o, o.dGradTab.ensure(tab.size() * sizeof(float)));
-        DH_CUDA(o, cudaMemcpyAsync(o.dGradTab.ptr, tab.data(), tab.size() * sizeof(float), cudaMemcpyHostToDevice, o.stream));
-        if (!fromWindow) {
-            const size_t winElems = (size_t)units * w * h;
-            DH_CUDA(o, o.dGradW.ensure(2 * winElems * sizeof(float2)));
-            float2* Wx = o.dGradW.as<float2>();
-            float2* Wy = Wx + winElems;
-            DH_CUDA(o, dh_launch_window_deriv(o.dWindow.as<float2>(), o.dGradTab.as<float>(), o.dGradTab.as<float>() + (size_t)P * w,
-                                              w, h, P, units, Wx, Wy, o.stream));
-            // fields of the derivative windows
-            DH_CUDA(o, o.dGradV.ensure(2 * (size_t)units * npix * sizeof(float2)));
-            Vx = o.dGradV.as<float2>();
-            Vy = Vx + (size_t)units * npix;
-            // both derivative windows in one launch: a batch of 2B frames (Wy follows Wx, Vy follows Vx)
-            DH_CUDA(o, o.dGradScratch.ensure(4 * (size_t)units * npix * sizeof(short) + (size_t)7 * P * (2 * B + 1) * sizeof(float)));
-            short* sR = o.dGradScratch.as<short>();
-            short* sI = sR + 2 * (size_t)units * npix;
-            float* sStats = reinterpret_cast<float*>(sI + 2 * (size_t)units * npix);
-            r = objInverseAux(o, Wx, 2 * B, Vx, sR, sI, sStats);
-            if (r) return r;
-        }
-        t2 = Clock::now();
-        // float modes up to order G + 1 (the waist derivative reaches m + 2)
-        const int GE = G + 2;
-        const int L = std::max(g.nx, g.ny);
-        DH_CUDA(o, o.dGradBasis.ensure((size_t)P * GE * (g.nx + g.ny) * sizeof(float) + (size_t)GE * L * sizeof(short) +
-                                       (size_t)GE * sizeof(float)));
-        hx = o.dGradBasis.as<float>();
-        hy = hx + (size_t)P * GE * g.nx;
-        float* scale = hy + (size_t)P * GE * g.ny;
-        short* s16 = reinterpret_cast<short*>(scale + GE);
-        r = objBasisFloat(o, GE, hx, hy, s16, scale);
-        if (r) return r;
-        t3 = Clock::now();
-    }
-
     gp.V = o.dField32.as<float2>();
-    gp.Vx = Vx;
-    gp.Vy = Vy;
     gp.coefs = o.dCoefs.as<float2>();
-    gp.hx = hx;
-    gp.hy = hy;
+    gp.weights = weights;
+    gp.out = out;
     gp.xAxis = o.dX.as<float>();
     gp.yAxis = o.dY.as<float>();
-    gp.nx = g.nx;
-    gp.ny = g.ny;
-    gp.frameCount = B;
-    gp.polCount = P;
-    gp.G = G;
-    gp.M = M;
+    gp.nx = o.geo.nx;
+    gp.ny = o.geo.ny;
+    gp.frameCount = o.batchCount;
+    gp.polCount = o.polCount;
+    gp.G = c.maxMG;
+    gp.M = o.modeCount;
     const float k0 = (float)(2.0 * PI_DA / c.wavelengthCentre);
-    for (int p = 0; p < P; p++) {
+    for (int p = 0; p < o.polCount; p++) {
         const int st = c.polLockTilt ? 0 : p;
         gp.k0u[p] = k0 * UNIT_ANGLE_A;
         gp.tiltX[p] = c.zern[st][ZERN_TILTX];
@@ -157,7 +87,184 @@ int objAlignEvaluate(Object& o, int metric, int stage, float* grad12, float* ilO
         gp.waist[p] = wv == 0 ? 400e-6f : wv;
     }
     gp.piOverLambda = (float)(PI_DA / c.wavelengthCentre);
+    return gp;
+}
+
+// Partial sums out[frame * P + pol][7] of the batch whose windows, fields,
+// coefficients and tables are on the device (frames of one wavelength).
+static int gradientSums(Object& o, bool fromWindow, const float2* weights, float* out, Clock::time_point& t2,
+                        Clock::time_point& t3) {
+    const Config& c = o.cfg;
+    const Geometry& g = o.geo;
+    const int P = o.polCount, B = o.batchCount, G = c.maxMG, M = o.modeCount;
+    const int units = B * P;
+    const int w = g.w, h = g.h, W = g.W, H = g.H;
+    const size_t npix = (size_t)g.nx * g.ny;
+    float2* Vx = nullptr;
+    float2* Vy = nullptr;
+    int r = ERR_SUCCESS;
+    // beam-centre phase derivatives of the window: i kx per column, i ky per row
+    std::vector<float> tab((size_t)P * (w + h));
+    for (int p = 0; p < P; p++) {
+        const int sx0 = g.SX[p] - W / 2;
+        for (int cc = 0; cc < w; cc++) tab[(size_t)p * w + cc] = g.kx[sx0 + cc];
+        for (int j = 0; j < h; j++) {
+            int row = (j + g.SY[p] + H / 2) % H;
+            if (row < 0) row += H;
+            tab[(size_t)P * w + (size_t)p * h + j] = g.ky[row];
+        }
+    }
+    DH_CUDA(o, o.dGradTab.ensure(tab.size() * sizeof(float)));
+    DH_CUDA(o, cudaMemcpyAsync(o.dGradTab.ptr, tab.data(), tab.size() * sizeof(float), cudaMemcpyHostToDevice, o.stream));
+    if (!fromWindow) {
+        const size_t winElems = (size_t)units * w * h;
+        DH_CUDA(o, o.dGradW.ensure(2 * winElems * sizeof(float2)));
+        float2* Wx = o.dGradW.as<float2>();
+        float2* Wy = Wx + winElems;
+        DH_CUDA(o, dh_launch_window_deriv(o.dWindow.as<float2>(), o.dGradTab.as<float>(), o.dGradTab.as<float>() + (size_t)P * w,
+                                          w, h, P, units, Wx, Wy, o.stream));
+        // fields of the derivative windows
+        DH_CUDA(o, o.dGradV.ensure(2 * (size_t)units * npix * sizeof(float2)));
+        Vx = o.dGradV.as<float2>();
+        Vy = Vx + (size_t)units * npix;
+        // both derivative windows in one launch: a batch of 2B frames (Wy follows Wx, Vy follows Vx)
+        DH_CUDA(o, o.dGradScratch.ensure(4 * (size_t)units * npix * sizeof(short) + (size_t)7 * P * (2 * B + 1) * sizeof(float)));
+        short* sR = o.dGradScratch.as<short>();
+        short* sI = sR + 2 * (size_t)units * npix;
+        float* sStats = reinterpret_cast<float*>(sI + 2 * (size_t)units * npix);
+        r = objInverseAux(o, Wx, 2 * B, Vx, sR, sI, sStats);
+        if (r) return r;
+    }
+    t2 = Clock::now();
+    // float modes up to order G + 1 (the waist derivative reaches m + 2)
+    const int GE = G + 2;
+    const int L = std::max(g.nx, g.ny);
+    DH_CUDA(o, o.dGradBasis.ensure((size_t)P * GE * (g.nx + g.ny) * sizeof(float) + (size_t)GE * L * sizeof(short) +
+                                   (size_t)GE * sizeof(float)));
+    float* hx = o.dGradBasis.as<float>();
+    float* hy = hx + (size_t)P * GE * g.nx;
+    float* scale = hy + (size_t)P * GE * g.ny;
+    short* s16 = reinterpret_cast<short*>(scale + GE);
+    r = objBasisFloat(o, GE, hx, hy, s16, scale);
+    if (r) return r;
+    t3 = Clock::now();
+    DhGradParams gp = gradientParams(o, weights, out);
+    gp.Vx = Vx;
+    gp.Vy = Vy;
+    gp.hx = hx;
+    gp.hy = hy;
+    if (!fromWindow) {
+        DH_CUDA(o, dh_launch_align_grad(gp, o.stream));
+        return ERR_SUCCESS;
+    }
+    DhGradWindowParams wp;
+    memset(&wp, 0, sizeof(wp));
+    DH_CUDA(o, o.dGradW.ensure(dh_grad_tables_elems(P, G, w, h) * sizeof(float2)));
+    wp.window = o.dWindow.as<float2>();
+    wp.coefs = gp.coefs;
+    wp.weights = gp.weights;
+    wp.hx = hx;
+    wp.hy = hy;
+    wp.refWaveF = o.dRefF.as<float>();
+    wp.xAxis = gp.xAxis;
+    wp.yAxis = gp.yAxis;
+    wp.kx = o.dGradTab.as<float>();
+    wp.ky = o.dGradTab.as<float>() + (size_t)P * w;
+    wp.twiddle = o.dTwiddle.as<float2>();
+    wp.tabX = o.dGradW.as<float2>();
+    wp.tabY = wp.tabX + (size_t)P * 5 * G * w;
+    auto log2of = [](int n) { int l = 0; while ((1 << l) < n) l++; return l; };
+    wp.w = w; wp.h = h; wp.logw = log2of(w); wp.logh = log2of(h);
+    wp.nx = g.nx; wp.ny = g.ny; wp.lognx = log2of(g.nx); wp.logny = log2of(g.ny);
+    wp.lowres = c.resolutionIdx;
+    wp.frameCount = B; wp.polCount = P; wp.G = G; wp.M = M;
+    for (int p = 0; p < P; p++) {
+        wp.sx0[p] = g.SX[p] - W / 2;
+        wp.sy[p] = g.SY[p];
+        wp.k0u[p] = gp.k0u[p];
+        wp.tiltX[p] = gp.tiltX[p];
+        wp.tiltY[p] = gp.tiltY[p];
+        wp.bcx[p] = gp.bcx[p];
+        wp.bcy[p] = gp.bcy[p];
+        wp.waist[p] = gp.waist[p];
+    }
+    wp.piOverLambda = gp.piOverLambda;
+    wp.out = gp.out;
+    DH_CUDA(o, dh_launch_align_grad_window(wp, o.stream));
+    return ERR_SUCCESS;
+}
+
+// The batch (of one or several wavelengths) with the gradient's sums of each
+// sub-batch of one wavelength taken while its windows, fields and tables are
+// on the device, into the rows of dGradOut where its outputs go.
+static int sweepGradient(Object& o, bool fromWindow, const float2* weights, Clock::time_point& t2, Clock::time_point& t3) {
+    const std::function<int(int, int, int)> visit = [&](int first, int step, int total) -> int {
+        int r = gradientShape(o);
+        if (r) return r;
+        const int S = o.batchCount, P = o.polCount, M = o.modeCount;
+        const size_t row = (size_t)P * M * sizeof(float2), sums = (size_t)P * 7 * sizeof(float);
+        DH_CUDA(o, o.dGradOut.ensure((size_t)total * sums));
+        DH_CUDA(o, o.dGradSub.ensure(S * (row + sums)));
+        float2* sub = o.dGradSub.as<float2>();
+        float* out = reinterpret_cast<float*>(o.dGradSub.as<char>() + S * row);
+        if (weights)
+            DH_CUDA(o, cudaMemcpy2DAsync(sub, row, weights + (size_t)first * P * M, step * row, row, S, cudaMemcpyDeviceToDevice,
+                                         o.stream));
+        r = gradientSums(o, fromWindow, weights ? sub : nullptr, out, t2, t3);
+        if (r) return r;
+        DH_CUDA(o, cudaMemcpy2DAsync(o.dGradOut.as<char>() + first * sums, step * sums, out, sums, sums, S,
+                                     cudaMemcpyDeviceToDevice, o.stream));
+        return ERR_SUCCESS;
+    };
+    struct Visit {
+        Object& o;
+        ~Visit() { o.sweepVisit = nullptr; }
+    } guard{o};
+    o.sweepVisit = &visit;
+    return objProcessForAlign(o);
+}
+
+// stage ALIGN_EVAL_FULL: the batch, the metric and its gradient;
+// ALIGN_EVAL_VALUE: the batch and the metric only (grad12 untouched);
+// ALIGN_EVAL_GRADIENT: the gradient (and the metric) of the batch state a
+// preceding ALIGN_EVAL_VALUE call left on the device, for the same metric.
+// The metric is the same number in every stage.  A batch of several
+// wavelengths runs as one sub-batch per wavelength, of which the device holds
+// the last one's windows and tables only: its gradient is taken within a
+// batch pass (for MDL, whose weights need all the coefficients, a second one).
+int objAlignEvaluate(Object& o, int metric, int stage, float* grad12, float* ilOut) {
+    Config& c = o.cfg;
+    if (c.maxMG <= 0) return fail(o, ERR_ERROR, "adjoint AutoAlign needs a modal basis (maxMG > 0)");
+    const auto t0 = Clock::now();
+    int r = ERR_SUCCESS;
+    const bool fromWindow = gradientFromWindow(o);
+    const bool valueOnly = stage == ALIGN_EVAL_VALUE;
+    bool sweep;
+    {
+        std::lock_guard<std::mutex> guard(o.lock);
+        objWavelengthUpdate(o);   // a pending array takes effect in this evaluation's batch
+        sweep = o.wavelengths.size() > 1;
+    }
+    struct Keep {
+        Object& o;
+        int keep;
+        ~Keep() { o.keepField32 = keep; }
+    } keep{o, o.keepField32};
+    if (!fromWindow || sweep) o.keepField32 = 1;
+    auto t1 = t0, t2 = t0, t3 = t0;
+    const bool within = sweep && !valueOnly && (stage == ALIGN_EVAL_GRADIENT || metric == 0);
+    if (within || stage != ALIGN_EVAL_GRADIENT) {
+        r = within ? sweepGradient(o, fromWindow, metric == 1 ? o.dGradWeights.as<float2>() : nullptr, t2, t3)
+                   : objProcessForAlign(o);
+        if (r) return r;
+    }
+    t1 = Clock::now();
+    r = gradientShape(o);
+    if (r) return r;
+    const int P = o.polCount, B = o.batchCount, M = o.modeCount;
+    const int units = B * P;
     double mdlDb = 0.0;
+    const float2* weights = nullptr;
     if (metric == 1) {
         // the weights of a value stage serve the gradient stage that follows it
         if (stage != ALIGN_EVAL_GRADIENT) {
@@ -167,53 +274,23 @@ int objAlignEvaluate(Object& o, int metric, int stage, float* grad12, float* ilO
             o.alignMdlDb = mdlDb;
         }
         mdlDb = o.alignMdlDb;
-        gp.weights = o.dGradWeights.as<float2>();
+        weights = o.dGradWeights.as<float2>();
     }
     DH_CUDA(o, o.dGradOut.ensure((size_t)units * 7 * sizeof(float)));
-    gp.out = o.dGradOut.as<float>();
+    float* sums = o.dGradOut.as<float>();
     if (valueOnly) {
-        DH_CUDA(o, dh_launch_align_power(gp, o.stream));
-    } else if (!fromWindow) {
-        DH_CUDA(o, dh_launch_align_grad(gp, o.stream));
-    } else {
-        DhGradWindowParams wp;
-        memset(&wp, 0, sizeof(wp));
-        DH_CUDA(o, o.dGradW.ensure(dh_grad_tables_elems(P, G, w, h) * sizeof(float2)));
-        wp.window = o.dWindow.as<float2>();
-        wp.coefs = gp.coefs;
-        wp.weights = gp.weights;
-        wp.hx = hx;
-        wp.hy = hy;
-        wp.refWaveF = o.dRefF.as<float>();
-        wp.xAxis = gp.xAxis;
-        wp.yAxis = gp.yAxis;
-        wp.kx = o.dGradTab.as<float>();
-        wp.ky = o.dGradTab.as<float>() + (size_t)P * w;
-        wp.twiddle = o.dTwiddle.as<float2>();
-        wp.tabX = o.dGradW.as<float2>();
-        wp.tabY = wp.tabX + (size_t)P * 5 * G * w;
-        auto log2of = [](int n) { int l = 0; while ((1 << l) < n) l++; return l; };
-        wp.w = w; wp.h = h; wp.logw = log2of(w); wp.logh = log2of(h);
-        wp.nx = g.nx; wp.ny = g.ny; wp.lognx = log2of(g.nx); wp.logny = log2of(g.ny);
-        wp.lowres = c.resolutionIdx;
-        wp.frameCount = B; wp.polCount = P; wp.G = G; wp.M = M;
-        for (int p = 0; p < P; p++) {
-            wp.sx0[p] = g.SX[p] - W / 2;
-            wp.sy[p] = g.SY[p];
-            wp.k0u[p] = gp.k0u[p];
-            wp.tiltX[p] = gp.tiltX[p];
-            wp.tiltY[p] = gp.tiltY[p];
-            wp.bcx[p] = gp.bcx[p];
-            wp.bcy[p] = gp.bcy[p];
-            wp.waist[p] = gp.waist[p];
-        }
-        wp.piOverLambda = gp.piOverLambda;
-        wp.out = gp.out;
-        DH_CUDA(o, dh_launch_align_grad_window(wp, o.stream));
+        DH_CUDA(o, dh_launch_align_power(gradientParams(o, weights, sums), o.stream));
+    } else if (!sweep) {
+        r = gradientSums(o, fromWindow, weights, sums, t2, t3);
+        if (r) return r;
+    } else if (!within) {
+        r = sweepGradient(o, fromWindow, weights, t2, t3);
+        if (r) return r;
+        sums = o.dGradOut.as<float>();
     }
     if (!o.hGradOut.ensure((size_t)units * 7 * sizeof(float))) return fail(o, ERR_MEMORYALLOCATION, "gradient host buffer");
     const float* part = o.hGradOut.as<float>();
-    DH_CUDA(o, cudaMemcpyAsync(o.hGradOut.ptr, gp.out, (size_t)units * 7 * sizeof(float), cudaMemcpyDeviceToHost, o.stream));
+    DH_CUDA(o, cudaMemcpyAsync(o.hGradOut.ptr, sums, (size_t)units * 7 * sizeof(float), cudaMemcpyDeviceToHost, o.stream));
     const auto t4 = Clock::now();
     DH_CUDA(o, cudaStreamSynchronize(o.stream));
     const auto t5 = Clock::now();

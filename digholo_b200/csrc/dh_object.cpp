@@ -1412,6 +1412,10 @@ static int processSweepLocked(Object& o, int syncCoefs) {
         if (r) return r;
         P = o.polCount; M = o.modeCount; nx = o.geo.nx; ny = o.geo.ny;
         active = o.basisActive; Mout = o.modeCountOut;
+        if (o.sweepVisit) {
+            r = (*o.sweepVisit)(outFast ? l : l * S, outFast ? L : 1, B);
+            if (r) return r;
+        }
         if (l == 0) {
             DH_CUDA(o, o.dAccCoefs.ensure((size_t)B * P * std::max(1, M) * sizeof(float2)));
             DH_CUDA(o, o.dAccCoefsOut.ensure((size_t)B * P * std::max(1, Mout) * sizeof(float2)));

@@ -7,6 +7,7 @@
 
 #include <cstddef>
 #include <cstdint>
+#include <functional>
 #include <mutex>
 #include <string>
 #include <memory>
@@ -191,7 +192,8 @@ struct Object {
     DevBuf dSnap[16];                   // AutoAlign parameter estimate: planes, sums, fields, tables
     DevBuf dTransRaw, dTransFrames;     // transposed uint16 input: raw host copy, converted frames
     // adjoint AutoAlign scratch: derivative windows and fields, float bases, partial sums
-    DevBuf dGradW, dGradV, dGradScratch, dGradBasis, dGradOut, dGradTab, dGradWeights;
+    // (dGradSub: weights and sums of one wavelength's sub-batch)
+    DevBuf dGradW, dGradV, dGradScratch, dGradBasis, dGradOut, dGradTab, dGradWeights, dGradSub;
     double alignMdlDb = 0.0;   // MDL of the batch state the MDL gradient weights belong to
     HostBuf hGradOut;
     DhEigen* eigen = nullptr;
@@ -249,6 +251,9 @@ struct Object {
     float sweepCentre = 0.f;
     const std::vector<float>* batchCalCaller = nullptr;
     int batchCalCallerCount = 0, batchCalCallerPol = 0;
+    // called for each sub-batch of it while the sub-batch is on the device:
+    // (first output row, row step, rows of the whole batch)
+    const std::function<int(int, int, int)>* sweepVisit = nullptr;
     // frames loaded by digHoloSetFrameBufferFromFile (owned, float32)
     std::vector<float> ownFrames;
     // digHoloConfigBackupSave / Load
