@@ -415,7 +415,6 @@ __global__ void __launch_bounds__(64 + 128 * NG, 1) k_forward_i8(const __grid_co
     static_assert(4 * NPAD * NB <= TMEMCOLS, "accumulator sets exceed tensor memory");
 
     extern __shared__ unsigned char smRaw[];
-    releaseDependent();
     unsigned char* base = reinterpret_cast<unsigned char*>(
         (reinterpret_cast<uintptr_t>(smRaw) + 1023) & ~static_cast<uintptr_t>(1023));
     const int GI = FUSE ? ip.maxMG : 0;
@@ -502,6 +501,10 @@ __global__ void __launch_bounds__(64 + 128 * NG, 1) k_forward_i8(const __grid_co
     __syncthreads();
     tc::fenceAfterSync();
     const uint32_t tmem = *tmemSlot;
+    // Only now that this block has its tensor memory: the dependent kernel may
+    // allocate some too (k_field128), and a block of it that took the columns
+    // first would wait for this kernel to end while this one waits for them.
+    releaseDependent();
 
     if (warp == 0) {
         // ---------------- TMA producer (the first `pre` tiles are out already)
