@@ -16,13 +16,23 @@ constexpr int TW_LOG = 12;
 // before the kernel ahead of it in the stream has ended; every thread calls
 // dependentWait before it touches what that kernel wrote (by plain loads: the
 // non-coherent ones may be moved across the wait).  Without the launch
-// attribute the wait returns at once.  releaseDependent, called by the kernel
-// ahead, lets the next one's blocks start as soon as this one's all have.  The
-// inverse kernels load their tables under the forward's tail: 16 frames of
-// 320 x 256 10.3 -> 8.2 us, 1024 of 640 x 512 34.3 -> 32.4.  Only the persistent
-// forward kernels release early: behind k_forward_win's partial last wave the
-// inverse's blocks would crowd on the SMs that come free first (131 us against
-// 127 without and 125 with the release at its blocks' ends).
+// attribute the wait returns at once.  The blocks start once all blocks ahead
+// have ended or called releaseDependent; their tables are then loaded under
+// the other kernel's tail.  16 frames of 320 x 256: 10.3 us without the
+// attribute, 8.2 with it and the early release.
+// Who releases early: the persistent forward kernels (DhFwdParams::releaseEarly),
+// - always, where the blocks behind fill an SM each (k_field128): they go where
+//   forward blocks end first, and nowhere else;
+// - where many small blocks follow (low-resolution fields, frame averaging),
+//   only while the forward blocks leave a third of the GPU free.  Otherwise the
+//   small blocks take the little room beside them, crowd there and end late:
+//   640 x 512 uint16, 32-pixel windows, one polarisation (148 forward blocks
+//   fill the GPU): 75 frames 21.5 us without the attribute, 19.6 released
+//   early, 20.1 at the blocks' ends; 147 frames 22.0, 31.8 and 20.1; 300
+//   frames 25.9, 33.9 and 24.1.
+// k_forward_win (127 us; released early 131, at its blocks' ends 125) and the
+// averaging kernel (100 items of two frames, 32-pixel windows: 10 % slower
+// released early) release at their blocks' ends.
 __device__ __forceinline__ void dependentWait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void releaseDependent() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

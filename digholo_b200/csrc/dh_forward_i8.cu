@@ -504,7 +504,7 @@ __global__ void __launch_bounds__(64 + 128 * NG, 1) k_forward_i8(const __grid_co
     // Only now that this block has its tensor memory: the dependent kernel may
     // allocate some too (k_field128), and a block of it that took the columns
     // first would wait for this kernel to end while this one waits for them.
-    releaseDependent();
+    if (p.releaseEarly) releaseDependent();
 
     if (warp == 0) {
         // ---------------- TMA producer (the first `pre` tiles are out already)
@@ -689,7 +689,9 @@ cudaError_t launchI8(const DhFwdParams& p, const DhInvParams& ip, const CUtensor
     int grid = sms < p.frameCount * P ? sms : p.frameCount * P;
     grid = (grid / P) * P;
     if (grid < P) grid = P;
-    kern<<<grid, 64 + 128 * NG, smem, s>>>(map, p, ip);
+    DhFwdParams q = p;
+    q.releaseEarly = p.wideFollower || 3 * p.frameCount * P <= 2 * sms;   // see dependentWait
+    kern<<<grid, 64 + 128 * NG, smem, s>>>(map, q, ip);
     return cudaGetLastError();
 }
 

@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(256, 2) k_forward_tma(const __grid_constant__ 
     constexpr int w = HW, h = HW;
     constexpr int Q = H / HW;
     extern __shared__ unsigned char smRaw[];
-    releaseDependent();
+    if (p.releaseEarly) releaseDependent();
     const int P = p.polCount;
     const int tid = threadIdx.x;
     constexpr unsigned tileBytes = (unsigned)H * ROWB;
@@ -341,7 +341,9 @@ cudaError_t launchTma(const DhFwdParams& p, const CUtensorMap& map, cudaStream_t
     if (perSM < 1) return cudaErrorNotSupported;
     const int units = p.frameCount * P;
     const int grid = units < perSM * smCountCached() ? units : perSM * smCountCached();
-    kern<<<grid, 2 * H, smem, s>>>(map, p);
+    DhFwdParams q = p;
+    q.releaseEarly = p.wideFollower || 3 * units <= 2 * perSM * smCountCached();   // see dependentWait
+    kern<<<grid, 2 * H, smem, s>>>(map, q);
     return cudaGetLastError();
 }
 

@@ -921,7 +921,6 @@ __global__ void __launch_bounds__(512) k_average_windows_reg(const float2* in, f
                                                              int batch, int avg, int mode, int polCount, int n,
                                                              const float2* __restrict__ cal, int calCount) {
     __shared__ double red[2][2][16];
-    releaseDependent();
     dependentWait();
     const int b = blockIdx.x / polCount, pol = blockIdx.x - b * polCount;
     const float inv = (float)(1.0 / avg);

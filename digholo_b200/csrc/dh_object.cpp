@@ -1040,6 +1040,7 @@ static int launchChunk(Object& o, const DhFwdParams& fp0, const DhInvParams& ip0
             cudaGetLastError();
         }
     }
+    fp.wideFollower = ip0.fieldR && !ip0.lowres;
     cudaError_t fe = launchForward(o, fp);
     if (fe != cudaSuccess) return failCuda(o, fe, "forward kernel launch");
     if (timed) DH_CUDA(o, cudaEventRecord(ev[1], o.stream));
