@@ -20,19 +20,10 @@ constexpr int TW_LOG = 12;
 // have ended or called releaseDependent; their tables are then loaded under
 // the other kernel's tail.  16 frames of 320 x 256: 10.3 us without the
 // attribute, 8.2 with it and the early release.
-// Who releases early: the persistent forward kernels (DhFwdParams::releaseEarly),
-// - always, where the blocks behind fill an SM each (k_field128): they go where
-//   forward blocks end first, and nowhere else;
-// - where many small blocks follow (low-resolution fields, frame averaging),
-//   only while the forward blocks leave a third of the GPU free.  Otherwise the
-//   small blocks take the little room beside them, crowd there and end late:
-//   640 x 512 uint16, 32-pixel windows, one polarisation (148 forward blocks
-//   fill the GPU): 75 frames 21.5 us without the attribute, 19.6 released
-//   early, 20.1 at the blocks' ends; 147 frames 22.0, 31.8 and 20.1; 300
-//   frames 25.9, 33.9 and 24.1.
-// k_forward_win (127 us; released early 131, at its blocks' ends 125) and the
-// averaging kernel (100 items of two frames, 32-pixel windows: 10 % slower
-// released early) release at their blocks' ends.
+// The persistent forward kernels release early where releasesEarly says so, the
+// averaging kernel before wide blocks.  Otherwise, and for k_forward_win always
+// (500 frames of 1280 x 1024: 127 us without the attribute, 131 released early,
+// 125 so), the release is the blocks' end.
 __device__ __forceinline__ void dependentWait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void releaseDependent() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -690,7 +690,7 @@ cudaError_t launchI8(const DhFwdParams& p, const DhInvParams& ip, const CUtensor
     grid = (grid / P) * P;
     if (grid < P) grid = P;
     DhFwdParams q = p;
-    q.releaseEarly = p.wideFollower || 3 * p.frameCount * P <= 2 * sms;   // see dependentWait
+    q.releaseEarly = releasesEarly(p, sms);
     kern<<<grid, 64 + 128 * NG, smem, s>>>(map, q, ip);
     return cudaGetLastError();
 }

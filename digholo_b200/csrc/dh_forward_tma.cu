@@ -342,7 +342,7 @@ cudaError_t launchTma(const DhFwdParams& p, const CUtensorMap& map, cudaStream_t
     const int units = p.frameCount * P;
     const int grid = units < perSM * smCountCached() ? units : perSM * smCountCached();
     DhFwdParams q = p;
-    q.releaseEarly = p.wideFollower || 3 * units <= 2 * perSM * smCountCached();   // see dependentWait
+    q.releaseEarly = releasesEarly(p, perSM * smCountCached());
     kern<<<grid, 2 * H, smem, s>>>(map, q);
     return cudaGetLastError();
 }

@@ -11,6 +11,8 @@
 #include <mutex>
 #include <utility>
 
+#include "dh_params.h"
+
 namespace dh {
 
 inline std::mutex& hostCacheLock() {
@@ -69,6 +71,24 @@ inline cudaError_t launchDependent(void (*kern)(Par...), unsigned grid, unsigned
     cfg.attrs = attr;
     cfg.numAttrs = early ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
+// Whether a persistent forward kernel with room for `capacity` blocks on the
+// GPU lets the kernel behind it start its blocks at once, instead of when its
+// own blocks have ended:
+// - where those blocks fill an SM each (k_field128): they go where forward
+//   blocks end first, and nowhere else;
+// - where they are small (low-resolution fields, averaging), while the forward
+//   leaves a third of its room free, or where they are so many (twelve units
+//   per SM) that they fill what room there is evenly.  In between they crowd
+//   beside the forward blocks or on the few free SMs and end late.
+// 640 x 512 uint16, 32-pixel windows, one polarisation (148 forward blocks fill
+// the GPU), us without the attribute / at the blocks' ends / at once: 75 frames
+// 21.5 / 20.1 / 19.6, 147 frames 22.0 / 20.1 / 31.8, 300 frames 25.9 / 24.1 /
+// 33.9; two polarisations: 500 frames 37.3 / 35.8 / 43.5, 800 frames 52.8 / 51.7
+// / 53.6, 1200 frames 74.2 / 73.2 / 70.4.
+inline bool releasesEarly(const DhFwdParams& p, int capacity) {
+    return p.wideFollower || 3ll * p.frameCount * p.polCount <= 2ll * capacity || p.followerUnits >= 12 * smCountCached();
 }
 
 inline PFN_cuTensorMapEncodeTiled_v12000 tensorMapEncoder() {

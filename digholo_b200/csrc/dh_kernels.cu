@@ -919,8 +919,9 @@ __global__ void __launch_bounds__(256) k_average_windows(const float2* __restric
 template <int AV>
 __global__ void __launch_bounds__(512) k_average_windows_reg(const float2* in, float2* __restrict__ out,
                                                              int batch, int avg, int mode, int polCount, int n,
-                                                             const float2* __restrict__ cal, int calCount) {
+                                                             const float2* __restrict__ cal, int calCount, int release) {
     __shared__ double red[2][2][16];
+    if (release) releaseDependent();   // only before blocks that fill an SM each (see dependentWait)
     dependentWait();
     const int b = blockIdx.x / polCount, pol = blockIdx.x - b * polCount;
     const float inv = (float)(1.0 / avg);
@@ -976,14 +977,16 @@ __global__ void __launch_bounds__(512) k_average_windows_reg(const float2* in, f
 }
 
 cudaError_t dh_launch_average_windows(const float2* in, float2* out, int batch, int avg, int mode, int polCount,
-                                      int n, const float2* cal, int calCount, int afterForward, cudaStream_t s) {
+                                      int n, const float2* cal, int calCount, int afterForward, int wideFollower,
+                                      cudaStream_t s) {
     if (batch <= 0 || polCount <= 0 || n <= 0) return cudaSuccess;
     if (avg < 1 || mode < 0 || mode > 2) return cudaErrorInvalidValue;
     if (n <= 512 * 8) {
         const int av = n <= 512 * 2 ? 2 : 8;   // two as far as 512 threads reach
         const int threads = (n + 32 * av - 1) / (32 * av) * 32;
         return launchDependent(av == 2 ? k_average_windows_reg<2> : k_average_windows_reg<8>, (unsigned)(batch * polCount),
-                               (unsigned)threads, 0, s, afterForward != 0, in, out, batch, avg, mode, polCount, n, cal, calCount);
+                               (unsigned)threads, 0, s, afterForward != 0, in, out, batch, avg, mode, polCount, n, cal, calCount,
+                               wideFollower);
     }
     k_average_windows<<<batch * polCount, 256, 0, s>>>(in, out, batch, avg, mode, polCount, n, cal, calCount);
     return cudaGetLastError();

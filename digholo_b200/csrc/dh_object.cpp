@@ -57,7 +57,8 @@ cudaError_t dh_launch_fields_to_c64(const short* R, const short* I, const float*
 cudaError_t dh_launch_batchsum(const short* R, const short* I, const float* stats, int statsStride,
                                int polCount, int frameCount, int npix, float* out, cudaStream_t s);
 cudaError_t dh_launch_average_windows(const float2* in, float2* out, int batch, int avg, int mode, int polCount,
-                                      int n, const float2* cal, int calCount, int afterForward, cudaStream_t s);
+                                      int n, const float2* cal, int calCount, int afterForward, int wideFollower,
+                                      cudaStream_t s);
 
 namespace dh {
 
@@ -1041,6 +1042,7 @@ static int launchChunk(Object& o, const DhFwdParams& fp0, const DhInvParams& ip0
         }
     }
     fp.wideFollower = ip0.fieldR && !ip0.lowres;
+    fp.followerUnits = (f1 - f0) * P;
     cudaError_t fe = launchForward(o, fp);
     if (fe != cudaSuccess) return failCuda(o, fe, "forward kernel launch");
     if (timed) DH_CUDA(o, cudaEventRecord(ev[1], o.stream));
@@ -1066,6 +1068,7 @@ static int launchAveraged(Object& o, const DhFwdParams& fp0, const DhInvParams& 
     fp.window = o.dWindowAvg.as<float2>();
     fp.batchCal = nullptr;   // per batch item, after the average
     fp.batchCalCount = 0;
+    fp.followerUnits = B * P;
     cudaEvent_t* ev = nullptr;
     if (o.timing) {
         if ((int)o.evStage.size() < 3 * (o.evStageUsed + 1)) {
@@ -1082,7 +1085,7 @@ static int launchAveraged(Object& o, const DhFwdParams& fp0, const DhInvParams& 
     cudaError_t fe = launchForward(o, fp);
     if (fe != cudaSuccess) return failCuda(o, fe, "forward kernel launch");
     DH_CUDA(o, dh_launch_average_windows(fp.window, fp0.window, B, A, o.cfg.avgMode, P, (int)n, fp0.batchCal,
-                                         fp0.batchCalCount, !ev, o.stream));
+                                         fp0.batchCalCount, !ev, ip.fieldR && !ip.lowres, o.stream));
     if (ev) DH_CUDA(o, cudaEventRecord(ev[1], o.stream));
     DhInvParams next = ip;
     next.afterForward = !ev;

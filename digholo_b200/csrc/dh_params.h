@@ -45,8 +45,9 @@ struct DhFwdParams {
     const unsigned char* dftDigits;
     int dftNpad;
     int* status;            // set to 1 by a kernel whose bounded wait expired (host-mapped)
-    int wideFollower;       // 1: the kernel behind this one has blocks that fill an SM each, 0: many small ones
-    int releaseEarly;       // the launcher's choice by it: start that kernel's blocks as this kernel's all run
+    int wideFollower;       // 1: the kernel behind this one has blocks that fill an SM each, 0: small ones
+    int followerUnits;      // units (frames x polarisations) that it has
+    int releaseEarly;       // the launcher's choice by them: start its blocks as this kernel's all run
 };
 
 // Inverse stage: Fourier window -> IFFT -> field statistics -> reference wave,
