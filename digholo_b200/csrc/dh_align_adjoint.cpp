@@ -32,6 +32,14 @@ enum { G_TX = 0, G_TY = 1, G_DEF = 2, G_CX = 3, G_CY = 4, G_WAIST = 5 };
 // pixels.  Otherwise it takes the float fields.
 static bool gradientFromWindow(const Object& o) { return !objRefCalApplies(o); }
 
+// Whether the next batch is one of several wavelengths (a pending array takes
+// effect in it).
+static bool severalWavelengths(Object& o) {
+    std::lock_guard<std::mutex> guard(o.lock);
+    objWavelengthUpdate(o);
+    return o.wavelengths.size() > 1;
+}
+
 // grad12[pol * 6 + k], k in {tiltX, tiltY, defocus, beamCentreX, beamCentreY,
 // waist} (config units: degrees, dioptre, m, m); parameters tied by the
 // polarisation locks carry the sum on polarisation 0 and zero on 1.
@@ -239,18 +247,13 @@ int objAlignEvaluate(Object& o, int metric, int stage, float* grad12, float* ilO
     int r = ERR_SUCCESS;
     const bool fromWindow = gradientFromWindow(o);
     const bool valueOnly = stage == ALIGN_EVAL_VALUE;
-    bool sweep;
-    {
-        std::lock_guard<std::mutex> guard(o.lock);
-        objWavelengthUpdate(o);   // a pending array takes effect in this evaluation's batch
-        sweep = o.wavelengths.size() > 1;
-    }
+    const bool sweep = severalWavelengths(o);
     struct Keep {
         Object& o;
-        int keep;
-        ~Keep() { o.keepField32 = keep; }
-    } keep{o, o.keepField32};
-    if (!fromWindow || sweep) o.keepField32 = 1;
+        int keep, defer;
+        ~Keep() { o.keepField32 = keep; o.deferField32 = defer; }
+    } keep{o, o.keepField32, o.deferField32};
+    (fromWindow && !sweep ? o.deferField32 : o.keepField32) = 1;
     auto t1 = t0, t2 = t0, t3 = t0;
     const bool within = sweep && !valueOnly && (stage == ALIGN_EVAL_GRADIENT || metric == 0);
     if (within || stage != ALIGN_EVAL_GRADIENT) {
@@ -390,9 +393,12 @@ float objAutoAlignAdjoint(Object& o) {
     const int userOnDevice = o.framesOnDevice;
     struct Restore {
         Object& o; const void* f; int d; int k;
-        ~Restore() { o.frames = f; o.framesOnDevice = d; o.keepField32 = k; o.useSnaps = 0; o.preparedValid = 0; }
+        ~Restore() {
+            o.frames = f; o.framesOnDevice = d; o.keepField32 = k; o.deferField32 = 0; o.useSnaps = 0; o.preparedValid = 0;
+        }
     } restore{o, userFrames, userOnDevice, o.keepField32};
-    if (!gradientFromWindow(o)) o.keepField32 = 1;   // every evaluation needs the float field for the adjoint
+    // every evaluation's float field, for the adjoint or for who asks for it afterwards
+    (gradientFromWindow(o) && !severalWavelengths(o) ? o.deferField32 : o.keepField32) = 1;
     {
         int r0 = objProcessForAlign(o);
         if (r0) return -FLT_MAX;

@@ -691,7 +691,7 @@ int digHoloB200SetKeepField32(int h, int enable) {
 // Copies the float fields of the last batch to host memory ([batch][pol][h][w]).
 complex64* digHoloB200GetFields32(int h, int* batchCount, int* polCount, int* width, int* height) {
     Object* o = get(h);
-    if (!o || !o->keepField32 || !o->processedTilt || !o->dField32.ptr) {
+    if (!o || !o->keepField32 || !o->processedTilt || dh::objDeferredField32(*o) != dh::ERR_SUCCESS || !o->dField32.ptr) {
         *batchCount = 0; *polCount = 0; *width = 0; *height = 0;
         return nullptr;
     }

@@ -574,6 +574,7 @@ static int prepare(Object& o) {
     if (r) return r;
     Config& c = o.cfg;
     if (!o.frames) return fail(o, ERR_NULLPOINTER, "frame buffer not set");
+    o.field32Deferred = 0;
     if (c.batchCount <= 0) c.batchCount = 1;
     o.batchCount = c.batchCount;
     o.avgCount = c.avgCount;
@@ -1700,6 +1701,8 @@ static int processBatchLocked(Object& o, int syncCoefs) {
     inverseParams(o, ip, 1);
     r = calParams(o, ip);
     if (r) return r;
+    o.field32Deferred = o.deferField32 && !ip.field32;
+    if (o.field32Deferred) o.deferredInv = ip;
     // the last stats column (aggregate over the batch) is filled on request
     if (o.avgCount > 1) {
         r = stageFrames(o, 0, B * o.avgCount, fp, 0);
@@ -1899,6 +1902,32 @@ int objInverseAux(Object& o, const float2* window, int frameCount, float2* field
     o.lastInverseKernel = k;
     o.lastOverlapKernel = ov;
     return ERR_SUCCESS;
+}
+
+// The float fields of the last batch where it left them (field32Deferred):
+// its inverse stage once more, on the windows it has left on the device.
+int objDeferredField32(Object& o) {
+    std::lock_guard<std::mutex> guard(o.lock);
+    if (!o.field32Deferred) return ERR_SUCCESS;
+    DhInvParams ip = o.deferredInv;
+    const int units = ip.frameCount * ip.polCount;
+    const size_t n = (size_t)units * o.geo.nx * o.geo.ny;
+    DH_CUDA(o, o.dField32.ensure(n * sizeof(float2)));
+    DH_CUDA(o, o.dGradScratch.ensure(2 * n * sizeof(short) + (size_t)ANALYSIS_COUNT * ip.polCount * ip.statsStride * sizeof(float)));
+    ip.field32 = o.dField32.as<float2>();
+    ip.fieldR = o.dGradScratch.as<short>();
+    ip.fieldI = ip.fieldR + n;
+    ip.stats = reinterpret_cast<float*>(ip.fieldI + n);
+    ip.fieldsOnly = 1;
+    ip.maxMG = ip.modeCount = 0;
+    ip.coefs = nullptr;
+    const int k = o.lastInverseKernel, ov = o.lastOverlapKernel;
+    DH_CUDA(o, launchInverse(o, ip));
+    o.lastInverseKernel = k;
+    o.lastOverlapKernel = ov;
+    DH_CUDA(o, cudaStreamSynchronize(o.stream));
+    o.field32Deferred = 0;
+    return objCheckStatus(o);
 }
 
 // Unquantised float HG modes [pol][modes][n] on the reconstructed-plane axes

@@ -176,6 +176,11 @@ struct Object {
     float basisPsx = 0.f, basisPsy = 0.f;
     int basisPolCount = 0;
     int keepField32 = 0;
+    // batches of the alignment gradient leave the float fields to be made from
+    // their windows when they are asked for: set while such batches run, and
+    // whether the last batch was one (with its inverse stage's parameters)
+    int deferField32 = 0, field32Deferred = 0;
+    DhInvParams deferredInv;
     // power meter / AutoAlign
     DevBuf dMetricA, dMetricG, dMetricW, dCoefsBackup, dAlignFrames;
     DevBuf dDigits;                     // tensor-core row DFT digits (uint16 frames)
@@ -299,6 +304,7 @@ int objWindowToHost(Object& o);
 int objStageTimes(Object& o, float* ms);
 int objUpdateBasis(Object& o);
 int objProcessForAlign(Object& o);
+int objDeferredField32(Object& o);
 int objCheckStatus(Object& o);
 void objReleaseGraphs(Object& o);
 // Kernel planner (plan modes above ESTIMATE): process-wide table of tuned
