@@ -29,8 +29,9 @@ enum { G_TX = 0, G_TY = 1, G_DEF = 2, G_CX = 3, G_CY = 4, G_WAIST = 5 };
 
 // The gradient takes the Fourier windows of the batch where the inverse stage
 // is separable: no reference-wave calibration, whose planes multiply the
-// pixels.  Otherwise it takes the float fields.
-static bool gradientFromWindow(const Object& o) { return !objRefCalApplies(o); }
+// pixels; and a field's coefficients fit the kernel's shared memory.  Otherwise
+// it takes the float fields.
+static bool gradientFromWindow(const Object& o) { return !objRefCalApplies(o) && dh_grad_window_fits(o.cfg.maxMG); }
 
 // Whether the next batch is one of several wavelengths (a pending array takes
 // effect in it).

@@ -805,6 +805,11 @@ cudaError_t dh_launch_align_grad(const DhGradParams& p, cudaStream_t s) {
 
 size_t dh_grad_tables_elems(int P, int G, int w, int h) { return (size_t)P * 5 * G * (w + h); }
 
+// The two coefficient tables [m][n] and [n][m]; 1 KB is left for the kernel's
+// own arrays.  Up to 120 groups.
+static size_t gradCoefBytes(int G) { return sizeof(float2) * 2 * (size_t)G * G; }
+bool dh_grad_window_fits(int G) { return gradCoefBytes(G) <= 226 * 1024; }
+
 // The refusal of the pixel kernels (fields whose row sums exceed shared
 // memory) holds here too: what can be aligned does not depend on a calibration.
 cudaError_t dh_launch_align_grad_window(const DhGradWindowParams& p, cudaStream_t s) {
@@ -813,7 +818,7 @@ cudaError_t dh_launch_align_grad_window(const DhGradWindowParams& p, cudaStream_
     const size_t any = sizeof(float2) * ((size_t)p.M + 2 * (size_t)p.G * p.ny) +
                        sizeof(float) * ((size_t)p.G * (p.nx + p.ny) + 8 * 7);
     if ((p.G > 32 || reg > 200 * 1024) && any > 200 * 1024) return cudaErrorNotSupported;
-    if (p.lognx > TW_LOG || p.logny > TW_LOG) return cudaErrorNotSupported;
+    if (p.lognx > TW_LOG || p.logny > TW_LOG || !dh_grad_window_fits(p.G)) return cudaErrorNotSupported;
     const size_t ts = 256 * 8 * sizeof(double) + (sizeof(double2) + sizeof(float4) + sizeof(float)) * (size_t)(p.nx > p.ny ? p.nx : p.ny);
     cudaError_t e = setSmemOnce(reinterpret_cast<const void*>(k_grad_tables), (int)ts);
     if (e != cudaSuccess) return e;
@@ -823,7 +828,7 @@ cudaError_t dh_launch_align_grad_window(const DhGradWindowParams& p, cudaStream_
     const unsigned units = (unsigned)(p.frameCount * p.polCount);
     // the base tables are read in pairs
     if ((reinterpret_cast<uintptr_t>(p.tabX) | reinterpret_cast<uintptr_t>(p.tabY)) & 15) return cudaErrorInvalidValue;
-    const size_t cs = sizeof(float2) * 2 * (size_t)p.G * p.G;
+    const size_t cs = gradCoefBytes(p.G);
     const size_t ws = cs + sizeof(float2) * ((size_t)p.h * (p.w + 1) + 5 * (size_t)p.G * (p.w + p.h));
     const bool sm = ws <= 200 * 1024;
     unsigned grid = (unsigned)smCountCached() * GB / p.polCount * p.polCount;

@@ -48,6 +48,8 @@ struct DhGradWindowParams {
     float* out;             // [unit][7], as in DhGradParams
 };
 size_t dh_grad_tables_elems(int polCount, int G, int w, int h);
+// Whether a field's coefficients for G mode groups fit the kernel's shared memory.
+bool dh_grad_window_fits(int G);
 cudaError_t dh_launch_align_grad_window(const DhGradWindowParams& p, cudaStream_t s);
 
 // Per field only the captured power sum |c|^2 into out[unit * 7 + 6] (the
