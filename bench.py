@@ -455,10 +455,9 @@ def main():
     w, hh, nx, ny = geo[2], geo[3], geo[4], geo[5]
     fwd_bytes = B * (P * W * H * 2 + P * w * hh * 8)
     inv_bytes = B * (P * w * hh * 8 + P * nx * ny * 4 + P * M * 8 + 7 * P * 4)
-    fwd_name = {1: "k_forward", 2: "k_forward_reg", 3: "k_forward_tma", 4: "k_forward_i8"}.get(
-        L.digHoloB200GetForwardKernel(h), "k_forward")
-    inv_name = {1: "k_inverse", 2: "k_inverse_lo16q" if w == 16 else "k_inverse_lo", 3: "k_field128" if nx == 128 and ny == 128 else "k_field_full",
-                4: "k_field_big"}.get(L.digHoloB200GetInverseKernel(h), "k_inverse")
+    fwd_name, inv_name = (L.digHoloB200GetKernelName(h, stage).decode() for stage in (0, 1))
+    if inv_name == "k_inverse_lo" and w == 16:
+        inv_name = "k_inverse_lo16q"
     if fwd_ms >= inv_ms:
         kname, kbytes, kms = fwd_name, fwd_bytes, fwd_ms / max(timed, 1)
     else:

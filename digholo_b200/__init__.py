@@ -54,6 +54,7 @@ def _bind_extensions(lib, out):
         "digHoloB200GetInverseKernel": (_C.c_int, [_C.c_int]),
         "digHoloB200SetOverlapKernel": (_C.c_int, [_C.c_int, _C.c_int]),
         "digHoloB200GetOverlapKernel": (_C.c_int, [_C.c_int]),
+        "digHoloB200GetKernelName": (_C.c_char_p, [_C.c_int, _C.c_int]),
         "digHoloB200AutoAlignGradient": (_C.c_int, [_C.c_int, P(_C.c_float), P(_C.c_float)]),
         "digHoloB200AutoAlignAdjoint": (_C.c_float, [_C.c_int]),
         "digHoloB200AutoAlignGradientMetric": (_C.c_int, [_C.c_int, _C.c_int, P(_C.c_float), P(_C.c_float)]),

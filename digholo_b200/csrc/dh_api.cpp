@@ -794,6 +794,12 @@ int digHoloB200GetForwardKernel(int h) {
     OBJ_OR(h, 0);
     return o->lastForwardKernel;
 }
+// The kernel itself that the last batch ran (stage 0 forward, 1 inverse), where
+// one number above stands for several; "" before the first batch.
+const char* digHoloB200GetKernelName(int h, int stage) {
+    OBJ_OR(h, "");
+    return stage == 0 ? o->lastForwardName : stage == 1 ? o->lastInverseName : "";
+}
 // Gradient of IL = 10 log10(sum |c|^2) + const with respect to
 // [pol][tiltX, tiltY, defocus, beamCentreX, beamCentreY, waist] at the current
 // configuration (Fourier-window selection held fixed), from one batch pass

@@ -801,19 +801,19 @@ static cudaError_t launchForward(Object& o, const DhFwdParams& fp, bool mayAlloc
     cudaError_t fe = cudaErrorNotSupported;
     if (mode == 0 || mode == 4) {
         fe = dh_launch_forward_i8(fp, o.stream);
-        if (fe == cudaSuccess) { o.lastForwardKernel = 4; return fe; }
+        if (fe == cudaSuccess) { o.lastForwardKernel = 4; o.lastForwardName = "k_forward_i8"; return fe; }
         if (fe != cudaErrorNotSupported || mode == 4) return fe;
         cudaGetLastError();
     }
     if (mode == 0 || mode == 3) {
         fe = dh_launch_forward_tma(fp, o.stream);
-        if (fe == cudaSuccess) { o.lastForwardKernel = 3; return fe; }
+        if (fe == cudaSuccess) { o.lastForwardKernel = 3; o.lastForwardName = "k_forward_tma"; return fe; }
         if (fe != cudaErrorNotSupported || mode == 3) return fe;
         cudaGetLastError();
     }
     if (mode == 0 || mode == 2) {
         fe = dh_launch_forward_reg(fp, o.stream);
-        if (fe == cudaSuccess) { o.lastForwardKernel = 2; return fe; }
+        if (fe == cudaSuccess) { o.lastForwardKernel = 2; o.lastForwardName = "k_forward_reg"; return fe; }
         if (fe != cudaErrorNotSupported || mode == 2) return fe;
         cudaGetLastError();
     }
@@ -822,7 +822,7 @@ static cudaError_t launchForward(Object& o, const DhFwdParams& fp, bool mayAlloc
     // planes (the plane buffer of the Fourier-plane requests, batch-sized)
     if ((mode == 0 && ((1 << fp.logW) >= 256 || !isPow2(fp.w) || !isPow2(fp.h))) || mode == 5) {
         fe = dh_launch_forward_win(fp, o.stream);
-        if (fe == cudaSuccess) { o.lastForwardKernel = 5; return fe; }
+        if (fe == cudaSuccess) { o.lastForwardKernel = 5; o.lastForwardName = "k_forward_win"; return fe; }
         if (fe != cudaErrorNotSupported) return fe;
         cudaGetLastError();
         const size_t Nx = (size_t)(1 << fp.logW) / 2 + 1;
@@ -836,12 +836,12 @@ static cudaError_t launchForward(Object& o, const DhFwdParams& fp, bool mayAlloc
         q.f = fp;
         q.plane = o.dFourier.as<float2>() + (size_t)fp.frameOffset * o.polCount * (1 << fp.logH) * Nx;
         fe = dh_launch_forward_plane(q, o.stream);
-        if (fe == cudaSuccess) { o.lastForwardKernel = 5; return fe; }
+        if (fe == cudaSuccess) { o.lastForwardKernel = 5; o.lastForwardName = "planes"; return fe; }
         if (fe != cudaErrorNotSupported || mode == 5) return fe;
         cudaGetLastError();
     }
     fe = dh_launch_forward(fp, o.stream);
-    if (fe == cudaSuccess) o.lastForwardKernel = 1;
+    if (fe == cudaSuccess) { o.lastForwardKernel = 1; o.lastForwardName = "k_forward"; }
     return fe;
 }
 
@@ -874,6 +874,7 @@ static cudaError_t launchBands(Object& o, const DhInvParams& ip, bool mayAlloc) 
         cudaError_t e = dh_launch_field512(ip, o.overlapKernel, o.dBigScratch.ptr, o.dBigScratch.bytes, &used, o.stream);
         if (e == cudaSuccess) {
             o.lastInverseKernel = 7;
+            o.lastInverseName = "k_field512";
             o.lastOverlapKernel = used;
             return e;
         }
@@ -891,6 +892,7 @@ static cudaError_t launchBands(Object& o, const DhInvParams& ip, bool mayAlloc) 
     cudaError_t e = dh_launch_field_big(ip, o.overlapKernel, o.dBigScratch.ptr, o.dBigScratch.bytes, &used, o.stream);
     if (e == cudaSuccess) {
         o.lastInverseKernel = 4;
+        o.lastInverseName = "k_field_big";
         o.lastOverlapKernel = used;
     }
     return e;
@@ -923,27 +925,28 @@ static cudaError_t launchInverse(Object& o, const DhInvParams& ip, bool mayAlloc
         // the calibration multiplies the IFFT output in the block-per-unit
         // kernels, or for larger full-resolution fields in k_field_big
         cudaError_t e = dh_launch_inverse(ip, o.stream);
-        if (e == cudaSuccess) { o.lastInverseKernel = 1; o.lastOverlapKernel = 1; return e; }
+        if (e == cudaSuccess) { o.lastInverseKernel = 1; o.lastInverseName = "k_inverse"; o.lastOverlapKernel = 1; return e; }
         if (e != cudaErrorNotSupported) return e;
         cudaGetLastError();
         if (!ip.lowres) return launchBands(o, ip, mayAlloc);   // k_field_big: fields beyond one block
         e = launchDft(o, ip, mayAlloc);
-        if (e == cudaSuccess) { o.lastInverseKernel = 6; o.lastOverlapKernel = 1; }
+        if (e == cudaSuccess) { o.lastInverseKernel = 6; o.lastInverseName = "k_inverse_dft"; o.lastOverlapKernel = 1; }
         return e;
     }
     if (o.inverseKernel == 2) return launchBands(o, ip, mayAlloc);
     if (o.inverseKernel == 0 || o.inverseKernel == 3) {   // 3: as 0 where not fused
         cudaError_t e = dh_launch_inverse_lo(ip, o.stream);
-        if (e == cudaSuccess) { o.lastInverseKernel = 2; o.lastOverlapKernel = 1; return e; }
+        if (e == cudaSuccess) { o.lastInverseKernel = 2; o.lastInverseName = "k_inverse_lo"; o.lastOverlapKernel = 1; return e; }
         if (e != cudaErrorNotSupported) return e;
         cudaGetLastError();
         // full resolution: field kernel, then the overlap kernel (128 x 128
         // fields with 48-pixel windows report the number of the band kernels,
         // whose folded transforms they run)
         const int fieldKernel = isPow2(ip.w) && isPow2(ip.h) ? 3 : 4;
+        const char* fieldName = ip.logW == 7 ? "k_field128" : "k_field_full";
         int fused = 0;
         e = dh_launch_field_full(ip, o.overlapKernel == 0, &fused, o.stream);
-        if (e == cudaSuccess && fused) { o.lastInverseKernel = fieldKernel; o.lastOverlapKernel = 2; return e; }
+        if (e == cudaSuccess && fused) { o.lastInverseKernel = fieldKernel; o.lastInverseName = fieldName; o.lastOverlapKernel = 2; return e; }
         if (e == cudaErrorNotSupported && fused) {
             cudaGetLastError();
             e = dh_launch_field_full(ip, 0, &fused, o.stream);
@@ -955,7 +958,7 @@ static cudaError_t launchInverse(Object& o, const DhInvParams& ip, bool mayAlloc
                 cudaGetLastError();
                 e = dh_launch_overlap_f32_chunked(ip, nx, ny, o.stream);
             }
-            if (e == cudaSuccess) { o.lastInverseKernel = fieldKernel; o.lastOverlapKernel = 1; return e; }
+            if (e == cudaSuccess) { o.lastInverseKernel = fieldKernel; o.lastInverseName = fieldName; o.lastOverlapKernel = 1; return e; }
             if (e != cudaErrorNotSupported) return e;
             cudaGetLastError();
             // overlap shape not covered: rerun the whole stage with another kernel
@@ -971,12 +974,12 @@ static cudaError_t launchInverse(Object& o, const DhInvParams& ip, bool mayAlloc
         }
     }
     cudaError_t e = dh_launch_inverse(ip, o.stream);
-    if (e == cudaSuccess) { o.lastInverseKernel = 1; o.lastOverlapKernel = 1; return e; }
+    if (e == cudaSuccess) { o.lastInverseKernel = 1; o.lastInverseName = "k_inverse"; o.lastOverlapKernel = 1; return e; }
     if (e != cudaErrorNotSupported || !ip.lowres) return e;
     // low-resolution fields whose sides are not powers of two
     cudaGetLastError();
     e = launchDft(o, ip, mayAlloc);
-    if (e == cudaSuccess) { o.lastInverseKernel = 6; o.lastOverlapKernel = 1; }
+    if (e == cudaSuccess) { o.lastInverseKernel = 6; o.lastInverseName = "k_inverse_dft"; o.lastOverlapKernel = 1; }
     return e;
 }
 
@@ -1031,6 +1034,7 @@ static int launchChunk(Object& o, const DhFwdParams& fp0, const DhInvParams& ip0
             if (fe == cudaSuccess) {
                 o.lastForwardKernel = 4;
                 o.lastInverseKernel = 5;
+                o.lastForwardName = o.lastInverseName = "k_forward_i8";
                 o.lastOverlapKernel = 1;
                 if (timed) {
                     DH_CUDA(o, cudaEventRecord(ev[1], o.stream));
@@ -1250,6 +1254,8 @@ static int launchBatchDevice(Object& o, const DhFwdParams& fp, const DhInvParams
         DH_CUDA(o, cudaGraphLaunch(g.exec, o.stream));
         o.lastForwardKernel = g.fwdKernel;
         o.lastInverseKernel = g.invKernel;
+        o.lastForwardName = g.fwdName;
+        o.lastInverseName = g.invName;
         o.lastOverlapKernel = g.ovlKernel;
         return ERR_SUCCESS;
     }
@@ -1289,6 +1295,8 @@ static int launchBatchDevice(Object& o, const DhFwdParams& fp, const DhInvParams
     g.exec = exec;
     g.fwdKernel = o.lastForwardKernel;
     g.invKernel = o.lastInverseKernel;
+    g.fwdName = o.lastForwardName;
+    g.invName = o.lastInverseName;
     g.ovlKernel = o.lastOverlapKernel;
     o.graphs.push_back(std::move(g));
     DH_CUDA(o, cudaGraphLaunch(exec, o.stream));
@@ -1898,8 +1906,10 @@ int objInverseAux(Object& o, const float2* window, int frameCount, float2* field
     ip.stats = scratchStats;
     ip.fieldsOnly = 1;
     const int k = o.lastInverseKernel, ov = o.lastOverlapKernel;
+    const char* name = o.lastInverseName;
     DH_CUDA(o, launchInverse(o, ip));
     o.lastInverseKernel = k;
+    o.lastInverseName = name;
     o.lastOverlapKernel = ov;
     return ERR_SUCCESS;
 }
@@ -1922,8 +1932,10 @@ int objDeferredField32(Object& o) {
     ip.maxMG = ip.modeCount = 0;
     ip.coefs = nullptr;
     const int k = o.lastInverseKernel, ov = o.lastOverlapKernel;
+    const char* name = o.lastInverseName;
     DH_CUDA(o, launchInverse(o, ip));
     o.lastInverseKernel = k;
+    o.lastInverseName = name;
     o.lastOverlapKernel = ov;
     DH_CUDA(o, cudaStreamSynchronize(o.stream));
     o.field32Deferred = 0;

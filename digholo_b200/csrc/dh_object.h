@@ -148,6 +148,7 @@ struct Object {
         std::vector<unsigned char> key;
         cudaGraphExec_t exec = nullptr;
         int fwdKernel = 0, invKernel = 0, ovlKernel = 0;
+        const char *fwdName = "", *invName = "";
     };
     std::vector<BatchGraph> graphs;
     std::vector<std::vector<unsigned char>> graphPending;   // settled argument sets (frame pointer zeroed)
@@ -211,6 +212,7 @@ struct Object {
     // generic), 1 generic, 2 register, 3 TMA-fed only; and the one that ran last
     int forwardKernel = 0;
     int lastForwardKernel = 0;
+    const char *lastForwardName = "", *lastInverseName = "";   // the kernels themselves
     // inverse kernel choice: 0 automatic (warp-per-unit kernel for 16/32-pixel
     // low-resolution fields, else the block kernel), 1 block kernel
     int inverseKernel = 0;

@@ -498,6 +498,12 @@ int digHoloB200SetOverlapKernel(int handleIdx, int kernel);
  * (512-wide fields). */
 int digHoloB200GetOverlapKernel(int handleIdx);
 
+/* The kernel itself that the last batch ran (testing aid), where one of the
+ * numbers above stands for several: stage 0 forward, 1 inverse. Forward 5 is
+ * "k_forward_win" or "planes"; inverse 3 "k_field128" or "k_field_full",
+ * inverse 4 "k_field128" or "k_field_big". "" before the first batch. */
+const char* digHoloB200GetKernelName(int handleIdx, int stage);
+
 /* Message of the handle's last error ("" when none). */
 const char* digHoloB200GetLastError(int handleIdx);
 
