@@ -958,7 +958,12 @@ static cudaError_t launchInverse(Object& o, const DhInvParams& ip, bool mayAlloc
                 cudaGetLastError();
                 e = dh_launch_overlap_f32_chunked(ip, nx, ny, o.stream);
             }
-            if (e == cudaSuccess) { o.lastInverseKernel = fieldKernel; o.lastInverseName = fieldName; o.lastOverlapKernel = 1; return e; }
+            if (e == cudaSuccess) {
+                o.lastInverseKernel = fieldKernel;
+                o.lastInverseName = fieldName;
+                o.lastOverlapKernel = fieldKernel == 4 && (ip.maxMG <= 0 || !ip.coefs) ? 0 : 1;   // 0: none, as the bands report it
+                return e;
+            }
             if (e != cudaErrorNotSupported) return e;
             cudaGetLastError();
             // overlap shape not covered: rerun the whole stage with another kernel

@@ -75,3 +75,17 @@ def test_bands_of_48_pixel_windows(lib, overlap):
     assert max(np.abs(g["R"].astype(int) - o["R"]).max(), np.abs(g["I"].astype(int) - o["I"]).max()) <= 2
     assert rel_l2(g["field"], o["field"]) <= 5e-5
     assert rel_l2(g["coefs"], o["coefs"]) <= (1e-4 if overlap == 0 else 5e-5)
+
+
+@pytest.mark.parametrize("inverse", [0, 2])
+def test_no_overlap_reported_without_modes(lib, inverse):
+    """48-pixel windows without a basis: overlap 0 from the field kernel as from the bands."""
+    hol = synth.generate(frame_count=2, frame_width=640, frame_height=512, pol_count=1, max_mg=3, waist=320e-6, snr_db=30,
+                         window=(128, 128), dtype="float32", seed=5, carrier=(0.6, 0.48))
+    h = lib.digHoloCreate()
+    api.configure(lib, h, config_for(hol, 0, max_mg=0))
+    assert lib.digHoloB200SetInverseKernel(h, inverse) == 0
+    api.run_batch(lib, h, hol.frames)
+    assert _names(lib, h)[1] == ("k_field_big" if inverse else "k_field128")
+    assert lib.digHoloB200GetInverseKernel(h) == 4 and lib.digHoloB200GetOverlapKernel(h) == 0
+    lib.digHoloDestroy(h)
