@@ -272,10 +272,10 @@ __global__ void __launch_bounds__(NT, 1) k_field512(DhInvParams p, F512Args a) {
     int4* refX = reinterpret_cast<int4*>(base + L.refX);
     float* red = reinterpret_cast<float*>(base + L.red);
     int* itemMN = reinterpret_cast<int*>(base + L.items);
-    uint64_t* bar = reinterpret_cast<uint64_t*>(base + L.misc);   // Hx load, products
-    uint32_t* tmemSlot = reinterpret_cast<uint32_t*>(bar + 2);
-    unsigned* passMax = reinterpret_cast<unsigned*>(bar + 3);     // [2] maxima of a band's passes (float bits)
-    unsigned long long& bandMax = *reinterpret_cast<unsigned long long*>(bar + 4);   // (maximum, index + 1)
+    uint64_t* bar = reinterpret_cast<uint64_t*>(base + L.misc);   // the products
+    uint32_t* tmemSlot = reinterpret_cast<uint32_t*>(bar + 1);
+    unsigned* passMax = reinterpret_cast<unsigned*>(bar + 2);     // [2] maxima of a band's passes (float bits)
+    unsigned long long& bandMax = *reinterpret_cast<unsigned long long*>(bar + 3);   // (maximum, index + 1)
 
     const int P = p.polCount, pol = blockIdx.x % P;   // the grid is a multiple of P
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(NT, 1) k_field512(DhInvParams p, F512Args a) {
         for (int e = tid; e < (G + 3) / 4 * 4 * HS; e += NT) hy[e] = 0.f;
         const uint4* src = reinterpret_cast<const uint4*>(a.hx + (size_t)pol * 8 * GN * 128);
         for (int e = tid; e < 8 * GN * 8; e += NT) reinterpret_cast<uint4*>(bop)[e] = __ldg(src + e);
-        if (tid == 0) tc::mbarInitTc(bar + 1);
+        if (tid == 0) tc::mbarInitTc(bar);
         if (warp == 0) {
             asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc::sAddr(tmemSlot)), "n"(TMCOLS)
                          : "memory");
@@ -607,7 +607,7 @@ __global__ void __launch_bounds__(NT, 1) k_field512(DhInvParams p, F512Args a) {
         }
         if (I8 && n > 0) {
             // the products of the previous pass have read the operand
-            ok = !__syncthreads_or(!tc::mbarWaitTc(bar + 1, (unsigned)((n - 1) & 1)));
+            ok = !__syncthreads_or(!tc::mbarWaitTc(bar, (unsigned)((n - 1) & 1)));
             if (!ok) break;
             readSums(par ^ 1);   // T of the band before has been contracted: its readers are past this barrier
         } else {
@@ -667,7 +667,7 @@ __global__ void __launch_bounds__(NT, 1) k_field512(DhInvParams p, F512Args a) {
                     tc::mmaI8(tmem + 4 * GN, ah, bl, tc::instrDescI8s(128, 2 * GN, true, false), k > 0);
                     tc::mmaI8(tmem + 6 * GN, ah, bh, tc::instrDescI8s(128, 2 * GN, true, true), k > 0);
                 }
-                tc::mmaCommit(bar + 1);
+                tc::mmaCommit(bar);
             }
             __syncwarp();
         } else if (par == 0 && n > 0) {
@@ -679,7 +679,7 @@ __global__ void __launch_bounds__(NT, 1) k_field512(DhInvParams p, F512Args a) {
     }
     if (I8) {
         if (ok && n > 0) {
-            ok = !__syncthreads_or(!tc::mbarWaitTc(bar + 1, (unsigned)((n - 1) & 1)));
+            ok = !__syncthreads_or(!tc::mbarWaitTc(bar, (unsigned)((n - 1) & 1)));
             if (ok) {
                 readSums((n - 1) & 1);
                 __syncthreads();
