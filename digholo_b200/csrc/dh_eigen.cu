@@ -776,11 +776,14 @@ cudaError_t launchHeevCluster(const HeevArgs& a, int count, cudaStream_t s) {
     return cudaLaunchKernelEx(&cfg, k_heev_cluster<Q, CC, CNT>, a);
 }
 
-// Shared memory holds the rows: of one block up to 64, of eight up to 304
-// (198 KB each).  128 threads a block up to n = 128, where the phase every
-// warp repeats is the longer one (metrics of 256 frames, n = 110: 480 us
-// against 493 with 256 threads); 256 beyond, where the rows
-// are (n = 240: 2415 us against 3148 with 128 and 2860 with 512).
+// Shared memory holds the rows: of one block up to n = 115, of eight up to 304
+// (216 KB each).  One block up to 64; beyond, eight are faster also where one
+// would do (metrics of 200 and 256 frames, n = 72 / 90 / 110: 237 / 279 / 354
+// us against 287 / 358 / 491 by one block).  128 threads a block up to n = 128,
+// where the phase every warp repeats is the longer one (metrics of 256 frames,
+// n = 110: 480 us against 493 with 256 threads, when the host's part still
+// followed the solver's); 256 beyond, where the rows are (n = 240: 2415 us
+// against 3148 with 128 and 2860 with 512).
 cudaError_t launchHeevFits(const HeevArgs& a, int count, cudaStream_t s) {
     const int n = a.n;
     if (n < 2 || n > 304 || count > 65535) return cudaErrorNotSupported;

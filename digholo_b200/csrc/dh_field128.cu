@@ -33,10 +33,10 @@
 // of N = 2 GN takes both), and the last mode row is the constant 1, whose sums
 // S undo the offset: T = sum F (Hx + 32768) - 32768 S.
 //
-// Bound: instruction issue (54 instructions per pixel, 46 % of the issue
-// slots; the rest is the phases' latency with four warps per scheduler).
-// 2048 units, 16-pixel windows, 15 groups: 119 us; 304 us with one block per
-// unit, scalar arithmetic (116 instructions per pixel) and bf16 products.
+// Bound: the phases' latency with four warps per scheduler (46 % of the issue
+// slots, 54 instructions per pixel).  2048 units, 16-pixel windows, 15 groups:
+// 110 us; 304 us with one block per unit, scalar arithmetic (116 instructions
+// per pixel) and bf16 products.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>

@@ -34,12 +34,12 @@
 // and its products run under the next pass's row transform.  Two passes' sums
 // are contracted with Hy in FP32; a last kernel sums the 64-row bands.
 //
-// Bound: instruction issue and the transforms' latency (44 % of the issue
-// slots in both passes with four warps per scheduler).  192 units of 512 x
-// 512, 30 groups: columns 27 us, statistics 94, quantising and overlap 215
-// (its global stores 11, the contraction 24, the products' issue 7); the band
-// kernels before, which repeated the column stage in each pass and used scalar
-// arithmetic, 190 and 340.
+// Bound: the transforms' latency (44 % of the issue slots in both passes with
+// four warps per scheduler).  192 units of 512 x 512, 30 groups: columns 25 us,
+// statistics 89, quantising and overlap 201 (its global stores 11, the
+// contraction 24, the products' issue 7); the band kernels before, which
+// repeated the column stage in each pass and used scalar arithmetic, 190 and
+// 340.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -68,7 +68,9 @@ __host__ __device__ constexpr int tPass(int GN) { return 4 * GN * TS + 16; }
 constexpr int APITCH = 64;    // buffered row of A (complex): column c at (c + sx0) mod 64, the others zero
 constexpr int GNMAX = 32;
 constexpr int ITEMS = 256;    // contraction items, at most 144 (32 mode groups), then end marks
-constexpr int CHUNK = 256;    // units whose column stage is held at a time
+// Units whose column stage is held at a time: at most 64 MiB, half of the L2,
+// since windows of up to 64 rows have w H <= 512 x 64.
+constexpr int CHUNK = 256;
 
 enum { P_STATS = 0, P_QUANT = 1, P_I8 = 2 };
 

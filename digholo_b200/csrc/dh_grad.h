@@ -24,8 +24,8 @@ struct DhGradParams {
     const float2* weights;
 };
 
-// The gradient from the Fourier windows (batches without a reference-wave
-// calibration): the scalars of DhGradParams and the separable pieces of the
+// The gradient from the Fourier windows (batches of one wavelength without a
+// reference-wave calibration, up to 120 mode groups): the scalars of DhGradParams and the separable pieces of the
 // inverse stage.
 struct DhGradWindowParams {
     const float2* window;   // [unit][h][w]

@@ -28,8 +28,9 @@ __global__ void k_gather_block(const float2* __restrict__ src0, const float2* __
 // A block has an 8 x 8 tile of G and four threads per element, each with a
 // quarter of every 64 terms; the quarters are added in a fixed order.  Bound:
 // the FP64 chain of a thread (K / 4 terms) and, at the sizes of a metrics
-// call, the number of blocks: 110 modes x 256 frames 26.6 us with one thread
-// per element in 16 x 16 tiles (49 blocks, 256 terms in a row), 10.2 us so.
+// call, the number of blocks: 110 modes x 256 frames 24.3 us with one thread
+// per element in 16 x 16 tiles (49 blocks, 256 terms in a row), 8.4 us so; 6 x
+// 40 5.9 and 3.4 us, 300 x 700 98 and 74, 600 x 700 293 and 259.
 constexpr int GT = 8, GK = 64;
 __global__ void __launch_bounds__(256) k_gram(const float2* __restrict__ A, int rows, int batch, int rowsGram,
                                               cuDoubleComplex* __restrict__ G) {

@@ -50,7 +50,7 @@ typedef float complex64[2];
 // the 8 MiB scratch (e.g. 2048 dual-polarisation frames with 16x16 IFFT
 // windows), and frameCount must not exceed the batch that call prepared
 // where that batch sized a scratch of the handle (the Fourier planes of
-// 256-pixel and wider windows, the band buffers of large full-resolution
+// windows beyond k_forward_win, the band buffers of large full-resolution
 // fields): larger calls return DIGHOLO_ERROR_MEMORYALLOCATION instead of
 // allocating.  The call makes the handle's device current (and leaves it
 // current); the first call on a device then looks up the scratch address on
