@@ -1924,6 +1924,7 @@ int objInverseAux(Object& o, const float2* window, int frameCount, float2* field
 int objDeferredField32(Object& o) {
     std::lock_guard<std::mutex> guard(o.lock);
     if (!o.field32Deferred) return ERR_SUCCESS;
+    cudaSetDevice(o.device);
     DhInvParams ip = o.deferredInv;
     const int units = ip.frameCount * ip.polCount;
     const size_t n = (size_t)units * o.geo.nx * o.geo.ny;
