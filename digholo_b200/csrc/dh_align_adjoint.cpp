@@ -57,9 +57,9 @@ int objAlignGradientMetric(Object& o, int metric, float* grad12, float* ilOut) {
 using Clock = std::chrono::steady_clock;
 
 // What a gradient needs of the last batch's geometry and basis.
+static bool powerOfTwoWindows(const Object& o) { return !((o.geo.w & (o.geo.w - 1)) || (o.geo.h & (o.geo.h - 1))); }
 static int gradientShape(Object& o) {
-    const Geometry& g = o.geo;
-    if ((g.w & (g.w - 1)) || (g.h & (g.h - 1)))
+    if (!powerOfTwoWindows(o))
         return fail(o, ERR_INVALIDDIMENSION, "the adjoint AutoAlign needs power-of-two IFFT window sides on this build");
     if (o.basisActive)
         return fail(o, ERR_INVALIDARGUMENT, "the adjoint AutoAlign works on Hermite-Gaussian coefficients (basis type 0)");
@@ -208,8 +208,7 @@ static int gradientSums(Object& o, bool fromWindow, const float2* weights, float
 // on the device, into the rows of dGradOut where its outputs go.
 static int sweepGradient(Object& o, bool fromWindow, const float2* weights, Clock::time_point& t2, Clock::time_point& t3) {
     const std::function<int(int, int, int)> visit = [&](int first, int step, int total) -> int {
-        int r = gradientShape(o);
-        if (r) return r;
+        if (!powerOfTwoWindows(o) || o.basisActive) return ERR_SUCCESS;   // refused once the batch is complete
         const int S = o.batchCount, P = o.polCount, M = o.modeCount;
         const size_t row = (size_t)P * M * sizeof(float2), sums = (size_t)P * 7 * sizeof(float);
         DH_CUDA(o, o.dGradOut.ensure((size_t)total * sums));
@@ -219,7 +218,7 @@ static int sweepGradient(Object& o, bool fromWindow, const float2* weights, Cloc
         if (weights)
             DH_CUDA(o, cudaMemcpy2DAsync(sub, row, weights + (size_t)first * P * M, step * row, row, S, cudaMemcpyDeviceToDevice,
                                          o.stream));
-        r = gradientSums(o, fromWindow, weights ? sub : nullptr, out, t2, t3);
+        const int r = gradientSums(o, fromWindow, weights ? sub : nullptr, out, t2, t3);
         if (r) return r;
         DH_CUDA(o, cudaMemcpy2DAsync(o.dGradOut.as<char>() + first * sums, step * sums, out, sums, sums, S,
                                      cudaMemcpyDeviceToDevice, o.stream));

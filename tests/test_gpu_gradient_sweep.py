@@ -113,3 +113,22 @@ def test_mdl_gradient_of_a_sweep(lib, orders):
     norm = np.linalg.norm(gf)
     assert ga @ gf / (np.linalg.norm(ga) * norm) >= 0.99
     assert np.abs(ga - gf).max() <= 0.05 * norm
+
+
+def test_refused_gradient_leaves_the_whole_batch(lib):
+    """A Laguerre-Gaussian output basis is refused after the batch, whose frames of all wavelengths stay."""
+    hol = _case(6)
+    cfg = _perturbed(hol, 0)
+    cfg.max_mg, cfg.basis_type = 4, 1
+    h, keep = _open(lib, cfg, hol.frames)
+    _wavelengths(lib, h, LAMBDA)
+    want = api.run_batch(lib, h, hol.frames)
+    g, il = (C.c_float * 12)(), C.c_float()
+    assert lib.digHoloB200AutoAlignGradient(h, g, C.byref(il)) == 8
+    b, m, p = C.c_int(), C.c_int(), C.c_int()
+    cp = lib.digHoloProcessBatch(h, C.byref(b), C.byref(m), C.byref(p))
+    lib.digHoloB200AutoAlignGradient(h, g, C.byref(il))
+    again = api.read_outputs(lib, h, 6, cp, m.value, p.value, True)
+    lib.digHoloDestroy(h)
+    assert again["R"].shape == want["R"].shape and np.array_equal(again["R"], want["R"])
+    assert np.array_equal(again["coefs"], want["coefs"])
