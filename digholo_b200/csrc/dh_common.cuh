@@ -21,7 +21,8 @@ constexpr int TW_LOG = 12;
 // the other kernel's tail.  16 frames of 320 x 256: 10.3 us without the
 // attribute, 8.2 with it and the early release.
 // The persistent forward kernels release early where releasesEarly says so, the
-// averaging kernel before wide blocks.  Otherwise, and for k_forward_win always
+// averaging kernel before blocks that fill an SM each or that fit beside the
+// forward kernel's.  Otherwise, and for k_forward_win always
 // (500 frames of 1280 x 1024: 127 us without the attribute, 131 released early,
 // 125 so), the release is the blocks' end.
 __device__ __forceinline__ void dependentWait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

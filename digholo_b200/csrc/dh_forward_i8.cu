@@ -690,7 +690,10 @@ cudaError_t launchI8(const DhFwdParams& p, const DhInvParams& ip, const CUtensor
     grid = (grid / P) * P;
     if (grid < P) grid = P;
     DhFwdParams q = p;
-    q.releaseEarly = releasesEarly(p, sms);
+    const DhFollower own = {grid, 64 + 128 * NG, regsCached(reinterpret_cast<const void*>(kern)), (int)smem};
+    q.releaseEarly = releasesEarly(p, own, 1);
+    if (p.own) *p.own = own;
+    q.own = nullptr;
     kern<<<grid, 64 + 128 * NG, smem, s>>>(map, q, ip);
     return cudaGetLastError();
 }

@@ -342,7 +342,10 @@ cudaError_t launchTma(const DhFwdParams& p, const CUtensorMap& map, cudaStream_t
     const int units = p.frameCount * P;
     const int grid = units < perSM * smCountCached() ? units : perSM * smCountCached();
     DhFwdParams q = p;
-    q.releaseEarly = releasesEarly(p, perSM * smCountCached());
+    const DhFollower own = {grid, 2 * H, regsCached(reinterpret_cast<const void*>(kern)), (int)smem};
+    q.releaseEarly = releasesEarly(p, own, perSM);
+    if (p.own) *p.own = own;
+    q.own = nullptr;
     kern<<<grid, 2 * H, smem, s>>>(map, q);
     return cudaGetLastError();
 }

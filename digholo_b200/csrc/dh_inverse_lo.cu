@@ -569,40 +569,49 @@ __global__ void __launch_bounds__(Q_THREADS) k_inverse_lo16q(DhInvParams p) {
     }
 }
 
-// Returns cudaErrorNotSupported for shapes this kernel does not cover.
-cudaError_t dh_launch_inverse_lo(const DhInvParams& p, cudaStream_t s) {
-    if (!p.lowres || p.logw != p.logh || (p.logw != 4 && p.logw != 5)) return cudaErrorNotSupported;
-    if (p.w != (1 << p.logw) || p.h != (1 << p.logh)) return cudaErrorNotSupported;   // power-of-two windows only
+// The launch of a shape the kernels cover: its blocks and their shared memory.
+static bool inverseLoShape(const DhInvParams& p, DhFollower& f) {
+    if (!p.lowres || p.logw != p.logh || (p.logw != 4 && p.logw != 5)) return false;
+    if (p.w != (1 << p.logw) || p.h != (1 << p.logh)) return false;   // power-of-two windows only
     // the table loads read 16-byte chunks of the int16 modes
-    if (p.maxMG > 0 && ((reinterpret_cast<uintptr_t>(p.hgX) | reinterpret_cast<uintptr_t>(p.hgY)) & 15))
-        return cudaErrorNotSupported;
+    if (p.maxMG > 0 && ((reinterpret_cast<uintptr_t>(p.hgX) | reinterpret_cast<uintptr_t>(p.hgY)) & 15)) return false;
     const int L = 1 << p.logw;
     const int units = p.frameCount * p.polCount;
-    if (units <= 0) return cudaSuccess;
     const int G = p.maxMG > 0 ? p.maxMG : 0;
     const int M = p.maxMG > 0 ? p.modeCount : 0;
     const int ULD = (G + 1) | 1;
-    const int UPB = (32 / L) * LO_WARPS;
     const size_t tables = sizeof(float) * ((size_t)2 * p.polCount * G * (L + 1) + L + 2 * (size_t)p.polCount * G) +
                           sizeof(int) * ((size_t)p.polCount * 4 * L + (size_t)((M + 1) & ~1));
+    const int UPB = L == 16 ? Q_UNITS : (32 / L) * LO_WARPS;
+    // tables, then at 16 pixels the statistics partials and per unit the row /
+    // field tile and U (tables is a multiple of 8 bytes: every count above is even)
+    const size_t smem = L == 16 ? tables + sizeof(float) * Q_UNITS * 2 * 8 + sizeof(float2) * (size_t)Q_UNITS * (L * Q_TLD + L * ULD)
+                                : tables + sizeof(float2) * (size_t)UPB * L * (ULD > L + 1 ? ULD : L + 1);
+    if (smem > 200 * 1024) return false;
+    f.blocks = (units + UPB - 1) / UPB;
+    f.threads = L == 16 ? Q_THREADS : 32 * LO_WARPS;
+    f.smem = (int)smem;
+    return true;
+}
+
+// The blocks dh_launch_inverse_lo would launch, with their registers (blocks 0:
+// it does not cover the shape).
+void dh_inverse_lo_blocks(const DhInvParams& p, DhFollower& f) {
+    f.blocks = 0;
+    if (!inverseLoShape(p, f)) return;
+    f.regs = regsCached(p.logw == 4 ? reinterpret_cast<const void*>(k_inverse_lo16q)
+                                    : reinterpret_cast<const void*>(k_inverse_lo<32>));
+}
+
+// Returns cudaErrorNotSupported for shapes this kernel does not cover.
+cudaError_t dh_launch_inverse_lo(const DhInvParams& p, cudaStream_t s) {
+    DhFollower f;
+    if (!inverseLoShape(p, f)) return cudaErrorNotSupported;
+    if (p.frameCount * p.polCount <= 0) return cudaSuccess;
     DhInvParams q = p;
-    q.maxMG = G;
-    q.modeCount = M;
-    cudaError_t e;
-    if (L == 16) {
-        // tables, the statistics partials, then per unit the row / field tile and U
-        // (tables is a multiple of 8 bytes: every count above is even)
-        const size_t smemQ = tables + sizeof(float) * Q_UNITS * 2 * 8 +
-                             sizeof(float2) * (size_t)Q_UNITS * (L * Q_TLD + L * ULD);
-        if (smemQ > 200 * 1024) return cudaErrorNotSupported;
-        e = setSmemOnce(reinterpret_cast<const void*>(k_inverse_lo16q), (int)smemQ);
-        if (e != cudaSuccess) return e;
-        return launchDependent(k_inverse_lo16q, (unsigned)((units + Q_UNITS - 1) / Q_UNITS), Q_THREADS, smemQ, s, p.afterForward != 0, q);
-    }
-    const size_t smem = tables + sizeof(float2) * (size_t)UPB * L * (ULD > L + 1 ? ULD : L + 1);
-    if (smem > 200 * 1024) return cudaErrorNotSupported;
-    const unsigned blocks = (unsigned)((units + UPB - 1) / UPB);
-    e = setSmemOnce(reinterpret_cast<const void*>(k_inverse_lo<32>), (int)smem);
+    if (q.maxMG <= 0) q.maxMG = q.modeCount = 0;
+    auto kern = p.logw == 4 ? k_inverse_lo16q : k_inverse_lo<32>;
+    const cudaError_t e = setSmemOnce(reinterpret_cast<const void*>(kern), f.smem);
     if (e != cudaSuccess) return e;
-    return launchDependent(k_inverse_lo<32>, blocks, 32 * LO_WARPS, smem, s, p.afterForward != 0, q);
+    return launchDependent(kern, (unsigned)f.blocks, (unsigned)f.threads, (size_t)f.smem, s, p.afterForward != 0, q);
 }

@@ -921,7 +921,7 @@ __global__ void __launch_bounds__(512) k_average_windows_reg(const float2* in, f
                                                              int batch, int avg, int mode, int polCount, int n,
                                                              const float2* __restrict__ cal, int calCount, int release) {
     __shared__ double red[2][2][16];
-    if (release) releaseDependent();   // only before blocks that fill an SM each (see dependentWait)
+    if (release) releaseDependent();
     dependentWait();
     const int b = blockIdx.x / polCount, pol = blockIdx.x - b * polCount;
     const float inv = (float)(1.0 / avg);
@@ -976,17 +976,35 @@ __global__ void __launch_bounds__(512) k_average_windows_reg(const float2* in, f
     }
 }
 
+static int averageThreads(int n, int& av) {
+    av = n <= 512 * 2 ? 2 : 8;   // two as far as 512 threads reach
+    return (n + 32 * av - 1) / (32 * av) * 32;
+}
+
+// The blocks dh_launch_average_windows would launch behind a forward kernel
+// (blocks 0: windows beyond the kernel that may start early).
+void dh_average_blocks(int batch, int polCount, int n, DhFollower& f) {
+    f.blocks = 0;
+    if (n > 512 * 8) return;
+    int av;
+    f.threads = averageThreads(n, av);
+    f.regs = regsCached(av == 2 ? reinterpret_cast<const void*>(k_average_windows_reg<2>)
+                                : reinterpret_cast<const void*>(k_average_windows_reg<8>));
+    f.smem = 512;
+    f.blocks = batch * polCount;
+}
+
 cudaError_t dh_launch_average_windows(const float2* in, float2* out, int batch, int avg, int mode, int polCount,
-                                      int n, const float2* cal, int calCount, int afterForward, int wideFollower,
+                                      int n, const float2* cal, int calCount, int afterForward, int release,
                                       cudaStream_t s) {
     if (batch <= 0 || polCount <= 0 || n <= 0) return cudaSuccess;
     if (avg < 1 || mode < 0 || mode > 2) return cudaErrorInvalidValue;
     if (n <= 512 * 8) {
-        const int av = n <= 512 * 2 ? 2 : 8;   // two as far as 512 threads reach
-        const int threads = (n + 32 * av - 1) / (32 * av) * 32;
+        int av;
+        const int threads = averageThreads(n, av);
         return launchDependent(av == 2 ? k_average_windows_reg<2> : k_average_windows_reg<8>, (unsigned)(batch * polCount),
                                (unsigned)threads, 0, s, afterForward != 0, in, out, batch, avg, mode, polCount, n, cal, calCount,
-                               wideFollower);
+                               release);
     }
     k_average_windows<<<batch * polCount, 256, 0, s>>>(in, out, batch, avg, mode, polCount, n, cal, calCount);
     return cudaGetLastError();

@@ -3,6 +3,8 @@
 // digHoloProcessBatch.
 #include "dh_object.h"
 
+#include "dh_host.h"
+
 #include <cuda_runtime.h>
 
 #include <atomic>
@@ -56,8 +58,10 @@ cudaError_t dh_launch_fields_to_c64(const short* R, const short* I, const float*
                                     int polCount, int frameCount, int npix, float2* out, cudaStream_t s);
 cudaError_t dh_launch_batchsum(const short* R, const short* I, const float* stats, int statsStride,
                                int polCount, int frameCount, int npix, float* out, cudaStream_t s);
+void dh_average_blocks(int batch, int polCount, int n, DhFollower& f);
+void dh_inverse_lo_blocks(const DhInvParams& p, DhFollower& f);
 cudaError_t dh_launch_average_windows(const float2* in, float2* out, int batch, int avg, int mode, int polCount,
-                                      int n, const float2* cal, int calCount, int afterForward, int wideFollower,
+                                      int n, const float2* cal, int calCount, int afterForward, int release,
                                       cudaStream_t s);
 
 namespace dh {
@@ -1053,6 +1057,7 @@ static int launchChunk(Object& o, const DhFwdParams& fp0, const DhInvParams& ip0
     }
     fp.wideFollower = ip0.fieldR && !ip0.lowres;
     fp.followerUnits = (f1 - f0) * P;
+    if (ip0.fieldR && ip0.lowres) dh_inverse_lo_blocks(ip, fp.follower);
     cudaError_t fe = launchForward(o, fp);
     if (fe != cudaSuccess) return failCuda(o, fe, "forward kernel launch");
     if (timed) DH_CUDA(o, cudaEventRecord(ev[1], o.stream));
@@ -1079,6 +1084,9 @@ static int launchAveraged(Object& o, const DhFwdParams& fp0, const DhInvParams& 
     fp.batchCal = nullptr;   // per batch item, after the average
     fp.batchCalCount = 0;
     fp.followerUnits = B * P;
+    dh_average_blocks(B, P, (int)n, fp.follower);
+    DhFollower own = {}, inverse = {};
+    fp.own = &own;
     cudaEvent_t* ev = nullptr;
     if (o.timing) {
         if ((int)o.evStage.size() < 3 * (o.evStageUsed + 1)) {
@@ -1094,8 +1102,12 @@ static int launchAveraged(Object& o, const DhFwdParams& fp0, const DhInvParams& 
     }
     cudaError_t fe = launchForward(o, fp);
     if (fe != cudaSuccess) return failCuda(o, fe, "forward kernel launch");
+    // the averaging kernel starts the inverse's blocks early where its own and
+    // they fit beside the forward kernel's, which can still be running then
+    if (ip.fieldR && ip.lowres) dh_inverse_lo_blocks(ip, inverse);
+    const int release = ip.fieldR && (!ip.lowres || bothFitBeside(own, fp.follower, inverse));
     DH_CUDA(o, dh_launch_average_windows(fp.window, fp0.window, B, A, o.cfg.avgMode, P, (int)n, fp0.batchCal,
-                                         fp0.batchCalCount, !ev, ip.fieldR && !ip.lowres, o.stream));
+                                         fp0.batchCalCount, !ev, release, o.stream));
     if (ev) DH_CUDA(o, cudaEventRecord(ev[1], o.stream));
     DhInvParams next = ip;
     next.afterForward = !ev;

@@ -5,6 +5,13 @@
 
 #define DH_MAXPOL 2
 
+// The blocks of a kernel launched behind another one: how many, and what each takes.
+struct DhFollower {
+    int blocks;             // 0: none that may start early
+    int threads, regs;      // per block, per thread
+    int smem;               // bytes per block
+};
+
 // Forward stage: frame window -> pruned R2C FFT -> Fourier window with the
 // reference's window operations (digHolo.cpp:6986-7260 and 1808-2122).
 struct DhFwdParams {
@@ -45,9 +52,11 @@ struct DhFwdParams {
     const unsigned char* dftDigits;
     int dftNpad;
     int* status;            // set to 1 by a kernel whose bounded wait expired (host-mapped)
-    int wideFollower;       // 1: the kernel behind this one has blocks that fill an SM each, 0: small ones
-    int followerUnits;      // units (frames x polarisations) that it has
+    int wideFollower;       // 1: the kernel behind this one has blocks that fill an SM each
+    DhFollower follower;    // else: its small blocks
+    int followerUnits;      // and its units (frames x polarisations)
     int releaseEarly;       // the launcher's choice by them: start its blocks as this kernel's all run
+    DhFollower* own;        // host: where a persistent kernel's launcher notes its own blocks, or null
 };
 
 // Inverse stage: Fourier window -> IFFT -> field statistics -> reference wave,
