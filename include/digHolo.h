@@ -431,7 +431,9 @@ int digHoloB200Synchronize(int handleIdx);
 int digHoloB200SetStream(int handleIdx, void* stream);
 
 /* Keep the float field -conj(A.ref) computed with the unquantised reference
- * wave, next to the int16 field; read it with digHoloB200GetFields32. */
+ * wave, next to the int16 field; read it with digHoloB200GetFields32.  After a
+ * gradient or an adjoint search the flag may also be set afterwards: the
+ * fields of its last batch are then made when they are read. */
 int digHoloB200SetKeepField32(int handleIdx, int enable);
 complex64* digHoloB200GetFields32(int handleIdx, int* batchCount, int* polCount, int* width, int* height);
 
@@ -577,7 +579,7 @@ int digHoloB200FrameSimulatorDevice(int frameCount, int frameWidth, int frameHei
  * digHoloB200ProcessBatchDevice first; that call allocates).  Sizes with
  * frameCount*polCount*w*h*8 bytes above 8 MiB are refused with
  * DIGHOLO_ERROR_INVALIDDIMENSION.  Where the preparing batch sized a scratch
- * of the handle (the Fourier planes of windows 256 pixels wide and more, the
+ * of the handle (the Fourier planes where a batch runs through them, the
  * band buffers of large full-resolution fields), a frameCount above that
  * batch's is refused with DIGHOLO_ERROR_MEMORYALLOCATION, not allocated.
  * The call makes the handle's device current and leaves it so; the first
